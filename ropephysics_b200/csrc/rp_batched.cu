@@ -253,7 +253,7 @@ __device__ void countSelfByBlocks(const RodView& V, const SelfScratch& S, int nS
 struct TeamCtx {
     RodGlobals G;                   // the rod's fixed global pointers (V.g)
     RodView V;                      // copies of the view and scratch for the
-    SelfScratch S;                  // separately compiled self-contact paths
+    SelfScratch S;                  // separately compiled paths
     int32_t* cursor;                // hash placement cursors (table entries)
     int32_t* partial;               // scan partials, one per warp
     int32_t* numLevels;             // projection levels of the pool
@@ -516,7 +516,8 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         G.force = A.force + R.pOff;
         G.kin = A.kinVel + R.pOff;
         G.torque = A.torque + R.sOff;
-        C.V = V;  // for the rarely run, separately compiled self-contact paths
+        C.V = V;  // for the rarely run, separately compiled paths
+        G.view = &C.V;
         C.S = S;
         C.partial = partial;
         C.numLevels = numLevels;

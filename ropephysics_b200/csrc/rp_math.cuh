@@ -79,6 +79,78 @@ __device__ __forceinline__ float norm2(V3 a) { return dot(a, a); }
 __device__ __forceinline__ float norm(V3 a) { return sqrtf(dot(a, a)); }
 __device__ __forceinline__ V3 cwise(V3 a, V3 b) { return V3{a.x * b.x, a.y * b.y, a.z * b.z}; }
 
+// ---------------------------------------------------------------- shared reciprocals
+//
+// The step's square roots and divisions are IEEE-rounded, and the dependent
+// chain of them (a 3x3 Cholesky solve is three roots and nine quotients) is
+// what one constraint projection waits for. The compiler's own sequences
+// each run their approximation, refinement and range branch anew; here the
+// divisors that repeat share one correctly rounded reciprocal, and one range
+// test at the end covers a whole projection:
+//   * root and reciprocal root come from one rsqrt approximation: one
+//     residual step for the root, one third-order step, y0 (1 + e + e^2) with
+//     e = 1 - s y0, for its reciprocal (the second-order one rounds two
+//     significands of s wrongly);
+//   * a / b with y = RN(1 / b): q = a y, r = a - q b (exact by FMA),
+//     RN(q + r y). This is Markstein's division step ("Computation of
+//     elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+//     Dev. 34(1), 1990), which rounds a / b correctly given the correctly
+//     rounded y. The residual is carried scaled by 2^64, so that it does not
+//     underflow: rods that move in a plane, or at one end, keep cross terms of
+//     1e-30 and less, down through the subnormals, and refusing those ran the
+//     fallback for every other warp of straight rods set in motion (0.92x).
+// Inside the ranges tested below the results equal sqrtf, 1 / x and a / b bit
+// for bit: the root and both reciprocals for every float of the range, the
+// quotient for every pair near enough to a rounding boundary to go wrong
+// (tests/test_gpu_shared_reciprocals.py). A subnormal quotient q - r y is off
+// by less than 2^-174 before its one rounding, and no quotient lies nearer a
+// boundary than that without lying on it: only an exact tie, a = b (2k + 1)
+// 2^-150, which needs an even integer b, could round to the other neighbour,
+// 2^-149 away. Outside the ranges -- NaN, infinities, singular matrices --
+// `ok` turns false and the caller falls back to the plain operators. Signs
+// of zero are kept too (b > 0).
+constexpr float kRootLo = 0x1p-64f, kRootHi = 0x1p64f;  // operands of sqrtRecip
+constexpr float kDivLo = 0x1p-32f, kDivHi = 0x1p32f;    // divisors
+
+// A divisor b > 0 and its reciprocal y = RN(1 / b), with the scaled pair that
+// the residual uses.
+struct Divisor {
+    float bS, y, yS;
+};
+__device__ __forceinline__ Divisor divisor(float b, float y) { return Divisor{b * 0x1p64f, y, y * 0x1p-64f}; }
+// s = sqrtf(a), y = 1 / s. A root with an all-ones significand is the one case
+// whose reciprocal the step rounds wrongly, to the power of two below it; it
+// is the common case of normalising a unit quaternion (s = 1 - 2^-24), so it is
+// mended here and not left to the fallback (0.48x on the grid of driven rods).
+__device__ __forceinline__ void sqrtRecip(float a, float& s, float& y, bool& ok) {
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(a));
+    const float s0 = a * y0;
+    s = fma3(fma3(-s0, s0, a), 0.5f * y0, s0);
+    const float e = fma3(-s, y0, 1.0f);
+    y = fma3(fma3(e, e, e), y0, y0);
+    y = __uint_as_float(__float_as_uint(y) + ((__float_as_uint(s) & 0x7fffffu) == 0x7fffffu ? 1u : 0u));
+    ok = ok & (a >= kRootLo) & (a <= kRootHi);
+}
+__device__ __forceinline__ Divisor rootDivisor(float a, bool& ok) {
+    float s, y;
+    sqrtRecip(a, s, y, ok);
+    return divisor(s, y);
+}
+// 1 / b for a positive b
+__device__ __forceinline__ float recip(float b, bool& ok) {
+    float y0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(b));
+    ok = ok & (b >= kDivLo) & (b <= kDivHi);
+    return fma3(fma3(-b, y0, 1.0f), y0, y0);
+}
+// a / b; the caller tests that what it computes from it stays finite
+// (|a| >= 2^64 overflows)
+__device__ __forceinline__ float quotient(float a, Divisor d) {
+    const float q = a * d.y;
+    return fma3(-fma3(q, d.bS, -(a * 0x1p64f)), d.yS, q);
+}
+
 __device__ __forceinline__ M3 mzero() {
     M3 r;
 #pragma unroll
@@ -158,6 +230,27 @@ __device__ __forceinline__ bool solveSPD3(const M3& A, V3 b, V3& y) {
     return true;
 }
 
+// The same solve with shared reciprocals; `ok` stays true only when the
+// result is solveSPD3's (which then returns true), bit for bit.
+__device__ __forceinline__ V3 solveSPD3Shared(const M3& A, V3 b, bool& ok) {
+    const Divisor l00 = rootDivisor(A.m[0][0], ok);
+    const float l10 = quotient(A.m[1][0], l00);
+    const float l20 = quotient(A.m[2][0], l00);
+    const Divisor l11 = rootDivisor(fma3(-l10, l10, A.m[1][1]), ok);
+    const float l21 = quotient(fma3(-l20, l10, A.m[2][1]), l11);
+    const Divisor l22 = rootDivisor(fma3(-l21, l21, fma3(-l20, l20, A.m[2][2])), ok);
+    const float z0 = quotient(b.x, l00);
+    const float z1 = quotient(fma3(-l10, z0, b.y), l11);
+    const float z2 = quotient(fma3(-l21, z1, fma3(-l20, z0, b.z)), l22);
+    V3 y;
+    y.z = quotient(z2, l22);
+    y.y = quotient(fma3(-l21, y.z, z1), l11);
+    y.x = quotient(fma3(-l20, y.z, fma3(-l10, y.y, z0)), l00);
+    // an overflow or NaN anywhere reaches y.x through the substitution
+    ok = ok & (fabsf(y.x) <= 0x1p100f);
+    return y;
+}
+
 __device__ __forceinline__ V3 im(Q4 q) { return V3{q.x, q.y, q.z}; }
 __device__ __forceinline__ Q4 qmake(float w, V3 v) { return Q4{w, v.x, v.y, v.z}; }
 __device__ __forceinline__ Q4 conj(Q4 q) { return Q4{q.w, -q.x, -q.y, -q.z}; }
@@ -196,6 +289,12 @@ __device__ __forceinline__ Q4 qnormalize(Q4 q) {
     const float n = sqrtf(qdot(q, q));
     return qscale(q, 1.0f / n);
 }
+// qnormalize with the shared root (see sqrtRecip)
+__device__ __forceinline__ Q4 qnormalizeShared(Q4 q, bool& ok) {
+    float s, y;
+    sqrtRecip(qdot(q, q), s, y, ok);
+    return qscale(q, y);
+}
 // body -> world: v + t w + u x t, t = 2 u x v
 __device__ __forceinline__ V3 rotate(Q4 q, V3 v) {
     const V3 u = im(q);
@@ -216,6 +315,13 @@ __device__ __forceinline__ Q4 applyBodyDelta(Q4 q, V3 theta) {
     const Q4 p = qmake(q.w - dot(av, bv), fmav(bv, q.w, av) + cross(av, bv));
     const float n = sqrtf(qdotB(p, p));
     return qscale(p, 1.0f / n);
+}
+__device__ __forceinline__ Q4 applyBodyDeltaShared(Q4 q, V3 theta, bool& ok) {
+    const V3 av = im(q), bv = theta * 0.5f;
+    const Q4 p = qmake(q.w - dot(av, bv), fmav(bv, q.w, av) + cross(av, bv));
+    float s, y;
+    sqrtRecip(qdotB(p, p), s, y, ok);
+    return qscale(p, y);
 }
 // Representative on the same hemisphere as the identity (the sign of w
 // decides; the reference's dot with the identity only adds zeros to it).

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
     const int tid = threadIdx.x, nth = blockDim.x;
 
     __shared__ RodGlobals sG;  // the rod's global pointers, read through V.g
+    __shared__ RodView sV;     // and its view, for the separately compiled paths
     RodGlobals G;
     RodView V = staticView(A, T, R, r, G);
     SelfScratch S;
@@ -144,9 +145,13 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
         S.overflow = reinterpret_cast<int32_t*>(smem + L.misc) + 2;
     }
     V.qComp = A.qComp + R.sOff;  // compensated frames: global in both forms
-    if (tid == 0) sG = G;
-    __syncthreads();
+    G.view = &sV;
     V.g = &sG;
+    if (tid == 0) {
+        sG = G;
+        sV = V;
+    }
+    __syncthreads();
     S.sorted = S.cellOf + nSt;
     S.segCount = S.sorted + nSt;
     S.segStart = S.segCount + nSt;

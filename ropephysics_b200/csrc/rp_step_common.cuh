@@ -42,6 +42,9 @@ struct RodGlobals {
     const float4* bComp;
     const float4* bRestD;
     const DPrim* prims;
+    // the rod's whole view, for the separately compiled fallbacks: a RodView
+    // passed to them by reference would have to leave the registers
+    const struct RodView* view;
 };
 
 struct RodView {
@@ -105,12 +108,23 @@ __device__ __forceinline__ V3 dispOf(const RodView& V, int i) {
 //
 // Frame j turned by the normalised body rotation (1, h)/|(1, h)| (h = half
 // the rotation vector, as applyBodyDelta and the frame prediction apply it).
-__device__ __forceinline__ void rotateFrameComp(const RodView& V, int j, V3 h) {
+// The rotation is (1, h)/s - 1 with s = |(1, h)|, 1/s - 1 written as
+// -t / (s (1 + s)), t = |h|^2, free of cancellation.
+__device__ __forceinline__ Q4 compRotation(V3 h) {
     const float t = norm2(h);
     const float s = sqrtf(1.0f + t);
     const float invS = 1.0f / s;
-    // (1, h)/s - 1, with 1/s - 1 = -t / (s (1 + s)) free of cancellation
-    const Q4 eu = qmake(-t / (s * (1.0f + s)), h * invS);
+    return qmake(-t / (s * (1.0f + s)), h * invS);
+}
+// The same with shared reciprocals (see sqrtRecip).
+__device__ __forceinline__ Q4 compRotationShared(V3 h, bool& ok) {
+    const float t = norm2(h);
+    float s, invS;
+    sqrtRecip(1.0f + t, s, invS, ok);
+    const float b = s * (1.0f + s);
+    return qmake(quotient(-t, divisor(b, recip(b, ok))), h * invS);
+}
+__device__ __forceinline__ void rotateFrameBy(const RodView& V, int j, Q4 eu) {
     const Q4 q = q4(V.q[j]);
     const Q4 c = q4(V.qComp[j]);
     const Q4 d = qsub(qmul(q, eu), qmul(c, eu));  // (q - c) (x) eu
@@ -120,6 +134,9 @@ __device__ __forceinline__ void rotateFrameComp(const RodView& V, int j, V3 h) {
     V.qComp[j] = f4(qsub(qsub(tq, q), y));
     const Q4 e = q4(V.qPrev[j]);  // (1 + e)(1 + eu) = 1 + e + eu + e eu
     V.qPrev[j] = f4(qadd(qadd(e, eu), qmul(e, eu)));
+}
+__device__ __forceinline__ void rotateFrameComp(const RodView& V, int j, V3 h) {
+    rotateFrameBy(V, j, compRotation(h));
 }
 
 // Rescale frame j's true quaternion q - qComp to unit length in FP64 and
@@ -139,18 +156,18 @@ __device__ __forceinline__ void renormalizeFrameComp(const RodView& V, int j) {
 // ---------------------------------------------------------------- constraints
 
 // Stretch constraint k between particles i0, i1 and frame j (the caller
-// passes sP0[k], sP1[k], sSeg[k], or k, k+1, k for a chain).
+// passes sP0[k], sP1[k], sSeg[k], or k, k+1, k for a chain), with the plain
+// operators: the fallback of projectStretchAt for what its shared
+// reciprocals do not cover. Not inlined, so that it costs the callers nothing.
 template <bool COMP>
-__device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0, int i1, int j, float invH2) {
+__device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int i0, int i1, int j, float invH2) {
+    const RodView& V = *g->view;
     const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
     const V3 iI = v3(V.g->invInertia[j]);
-    if (w0 == 0.0f && w1 == 0.0f && norm2(iI) == 0.0f) return;
-
     const float4 sc = V.g->sComp[k];
     const float l = sc.w;
     const Q4 q = q4(V.q[j]);
     V3 d = v3(V.x[i1]) - v3(V.x[i0]);
-    // compensated mode: the segment vector of the true (x - xComp) positions
     if (COMP) d = d - (v3(V.xComp[i1]) - v3(V.xComp[i0]));
     const V3 u = divs(rotateInv(q, d), l);
     const V3 C = u - V3{0.0f, 0.0f, 1.0f};
@@ -161,8 +178,6 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     A.m[1][1] += alpha.y;
     A.m[2][2] += alpha.z;
 
-    // no multiplier array: one iteration, so this projection is the
-    // constraint's only one of the substep and its multiplier starts at zero
     const V3 lam = V.lamS ? v3(V.lamS[k]) : V3{0.0f, 0.0f, 0.0f};
     V3 dL;
     if (!solveSPD3(A, -fmacw(alpha, lam, C), dL)) return;
@@ -180,18 +195,80 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     }
 }
 
+// The same projection, bit for bit, with shared reciprocals: everything is
+// computed and range-tested before the first write, and what the test
+// refuses runs projectStretchPlain instead.
+//
+// Bound: the latency of one dependent FP32 chain per constraint (four colours
+// of them per sweep, one to four warps per scheduler); the plain operators
+// made 14 of its steps divisions and 4 of them roots. Plain -> shared, whole
+// steps on a B200: one 64-segment cantilever, 20 substeps, 253 -> 178 us;
+// 4096 driven rods of 64, 80 substeps, 1.82 -> 1.30 ms; 777 rods of 97, 8
+// substeps x 3 sweeps, compensated, 194 -> 147 us; 4096 uneven rods, 50
+// substeps, self-collision on, 8.80 -> 7.77 ms.
+template <bool COMP>
+__device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0, int i1, int j, float invH2) {
+    const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
+    const V3 iI = v3(V.g->invInertia[j]);
+    if (w0 == 0.0f && w1 == 0.0f && norm2(iI) == 0.0f) return;
+
+    bool ok = true;
+    const float4 sc = V.g->sComp[k];
+    const float l = sc.w;
+    const float invL = recip(l, ok);
+    const Q4 q = q4(V.q[j]);
+    V3 d = v3(V.x[i1]) - v3(V.x[i0]);
+    // compensated mode: the segment vector of the true (x - xComp) positions
+    if (COMP) d = d - (v3(V.xComp[i1]) - v3(V.xComp[i0]));
+    const V3 u = rotateInv(q, d) * invL;
+    const V3 C = u - V3{0.0f, 0.0f, 1.0f};
+
+    const V3 alpha = v3(sc) * (invH2 * V.complianceScale);
+    const Divisor dl = divisor(l, invL);
+    const float ll = l * l;
+    const float wl = quotient(w0 + w1, divisor(ll, recip(ll, ok)));
+    const float s0 = quotient(w0, dl), s1 = quotient(w1, dl);
+    ok = ok & (fmaxf(fabsf(w0), fabsf(w1)) <= 0x1p60f);
+    M3 A = madd(midentity(wl), sandwichDiag<true>(mskew(u), iI));
+    A.m[0][0] += alpha.x;
+    A.m[1][1] += alpha.y;
+    A.m[2][2] += alpha.z;
+
+    // no multiplier array: one iteration, so this projection is the
+    // constraint's only one of the substep and its multiplier starts at zero
+    const V3 lam = V.lamS ? v3(V.lamS[k]) : V3{0.0f, 0.0f, 0.0f};
+    const V3 dL = solveSPD3Shared(A, -fmacw(alpha, lam, C), ok);
+
+    const V3 world = rotate(q, dL);
+    const V3 theta = cwise(iI, cross(dL, u));
+    const Q4 turned = COMP ? compRotationShared(theta * 0.5f, ok) : applyBodyDeltaShared(q, theta, ok);
+    if (!ok) {
+        projectStretchPlain<COMP>(V.g, k, i0, i1, j, invH2);
+        return;
+    }
+    if (V.lamS) V.lamS[k] = f4(lam + dL);
+    addPos<COMP>(V, i0, -world, s0);
+    addPos<COMP>(V, i1, world, s1);
+    if (norm2(iI) > 0.0f) {
+        if (COMP)
+            rotateFrameBy(V, j, turned);
+        else
+            V.q[j] = f4(turned);
+    }
+}
+
 template <bool COMP>
 __device__ __forceinline__ void projectStretchOne(const RodView& V, int k, float invH2) {
     projectStretchAt<COMP>(V, k, V.g->sP0[k], V.g->sP1[k], V.g->sSeg[k], invH2);
 }
 
 // Bend/twist constraint k between frames a and b (bA[k], bB[k], or k, k+1
-// for a chain's real frames).
+// for a chain's real frames) with the plain operators: the fallback of
+// projectBendAt.
 template <bool COMP>
-__device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, int b, float invH2) {
+__device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a, int b, float invH2) {
+    const RodView& V = *g0->view;
     const V3 iIa = v3(V.g->invInertia[a]), iIb = v3(V.g->invInertia[b]);
-    if (norm2(iIa) == 0.0f && norm2(iIb) == 0.0f) return;
-
     const float4 bc = V.g->bComp[k];
     const float lbar = bc.w;
     const Q4 qa = q4(V.q[a]);
@@ -227,6 +304,59 @@ __device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, in
             rotateFrameComp(V, b, cwise(iIb, g) * 0.5f);
         else
             V.q[b] = f4(applyBodyDelta(qb, cwise(iIb, g)));
+    }
+}
+
+// The same projection, bit for bit, with shared reciprocals (see
+// projectStretchAt).
+template <bool COMP>
+__device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, int b, float invH2) {
+    const V3 iIa = v3(V.g->invInertia[a]), iIb = v3(V.g->invInertia[b]);
+    if (norm2(iIa) == 0.0f && norm2(iIb) == 0.0f) return;
+
+    bool ok = true;
+    const float4 bc = V.g->bComp[k];
+    const float invL = recip(bc.w, ok);
+    const Q4 qa = q4(V.q[a]);
+    const Q4 qb = q4(V.q[b]);
+    const Q4 p = sameHemisphereId(qmulConj(qa, qb));
+    // 2 / l is 2 (1 / l) exactly
+    const V3 C = fmav(im(p), 2.0f * invL, -v3(V.g->bRestD[k]));
+
+    const M3 skewPv = mskew(im(p));
+    const M3 Ja = mscale(madd(midentity(-p.w), skewPv), invL);
+    const M3 Jb = mscale(madd(midentity(p.w), skewPv), invL);
+
+    const V3 alpha = v3(bc) * (invH2 * V.complianceScale);
+    M3 A = madd(sandwichDiag<false>(Ja, iIa), sandwichDiag<false>(Jb, iIb));
+    A.m[0][0] += alpha.x;
+    A.m[1][1] += alpha.y;
+    A.m[2][2] += alpha.z;
+
+    const V3 lam = V.lamB ? v3(V.lamB[k]) : V3{0.0f, 0.0f, 0.0f};
+    const V3 dL = solveSPD3Shared(A, -fmacw(alpha, lam, C), ok);
+
+    const V3 side = cross(im(p), dL);
+    const V3 ta = cwise(iIa, fmav(dL, -p.w, -side) * invL);
+    const V3 tb = cwise(iIb, fmav(dL, p.w, -side) * invL);
+    const Q4 ra = COMP ? compRotationShared(ta * 0.5f, ok) : applyBodyDeltaShared(qa, ta, ok);
+    const Q4 rb = COMP ? compRotationShared(tb * 0.5f, ok) : applyBodyDeltaShared(qb, tb, ok);
+    if (!ok) {
+        projectBendPlain<COMP>(V.g, k, a, b, invH2);
+        return;
+    }
+    if (V.lamB) V.lamB[k] = f4(lam + dL);
+    if (norm2(iIa) > 0.0f) {
+        if (COMP)
+            rotateFrameBy(V, a, ra);
+        else
+            V.q[a] = f4(ra);
+    }
+    if (norm2(iIb) > 0.0f) {
+        if (COMP)
+            rotateFrameBy(V, b, rb);
+        else
+            V.q[b] = f4(rb);
     }
 }
 
@@ -684,10 +814,18 @@ __device__ __forceinline__ void predictFrameFrom(const RodView& V, int j, float 
     const V3 tau = rotateInv(q, v3(V.g->torque[j]));
     const V3 wn = fmav(cwise(iI, tau - cross(w, cwise(v3(V.g->inertia[j]), w))), h, w);
     if (wOut) *wOut = f4(wn);
-    if (COMP)
-        rotateFrameComp(V, j, wn * (0.5f * h));
-    else
-        V.q[j] = f4(qnormalize(qfma(qmul(q, qmake(0.0f, wn)), 0.5f * h, q)));
+    bool ok = true;
+    if (COMP) {
+        const V3 half = wn * (0.5f * h);
+        Q4 eu = compRotationShared(half, ok);
+        if (!ok) eu = compRotation(half);
+        rotateFrameBy(V, j, eu);
+    } else {
+        const Q4 p = qfma(qmul(q, qmake(0.0f, wn)), 0.5f * h, q);
+        Q4 n = qnormalizeShared(p, ok);
+        if (!ok) n = qnormalize(p);
+        V.q[j] = f4(n);
+    }
 }
 
 template <bool COMP>
