@@ -22,11 +22,13 @@
 //     tighter than the per-pair sphere test, then the per-pair test and the
 //     shared narrow phase), each weighted by that multiplicity: the same
 //     counts, without building the hash when nothing touches;
-//   * when something touches, the hash is built (stable counting sort: team
-//     scans and one warp placing segments in order with __match_any_sync) and
-//     the reference's fill pass writes the pool in its exact order;
+//   * when something touches, the pool is built from the touching pairs in
+//     the reference's order: each entry's place is counted among its
+//     segment's pairs. Only with more pairs than segments is the reference's
+//     hash built (stable counting sort) and its fill pass run;
 //   * the pool is projected level by level (contacts of a level share no
-//     particle), which reproduces the sequential order's arithmetic.
+//     particle), which reproduces the sequential order's arithmetic, from
+//     shared memory and by one warp while levels are narrow.
 // Every per-element operation is the shared code in rp_step_common.cuh, so
 // results are bit-identical to the plain kernel.
 #include <cuda_runtime.h>
@@ -123,15 +125,47 @@ __device__ __forceinline__ unsigned bucketCells(float4 cj, float4 ck, float cell
     return m;
 }
 
-// Multiplicity of a touching pair in the reference's count: the number of
-// the 27 cells around cell(j) whose hash is k's bucket hash(cell(k)).
-__device__ __forceinline__ int bucketMultiplicity(float4 cj, float4 ck, float cell, int table) {
-    return __popc(bucketCells(cj, ck, cell, table));
-}
+// What a team needs about its rod beyond its shared-memory arrays: the fixed
+// global pointers, the colour tables, the drive, the self-contact scratch.
+// Lane 0 writes it once per rod into shared memory and every phase reads the
+// fields it uses, so the substep loop carries only the current phase's values
+// in registers (held in registers, these 64-bit pointers filled a third of
+// the register file and pushed the constraint arithmetic into spills). The
+// arrays in shared memory are not reached through it: pointers read back
+// from memory lose their address space, and every access through them
+// would be a generic load.
+struct TeamCtx {
+    RodGlobals G;                   // the rod's fixed global pointers (V.g)
+    RodView V;                      // copies of the view and scratch for the
+    SelfScratch S;                  // separately compiled paths
+    const int* sOrder;
+    const int* bOrder;
+    const int* sCol;
+    const int* bCol;
+    int32_t nP, nSt;
+    int32_t table, selfGap, selfCapacity;
+    float selfFriction;
+    double tRod;                    // the rod's simulated time (lane 0 advances it)
+    int32_t driveP, wayP, wayStep;  // driven particle, waypoint particle and step
+    int32_t stageFailed;            // a lane gave up waiting for the staged state
+    uint64_t bar;                   // mbarrier of the rod's bulk stage-in
+
+    // the rod's misc words (rp_layout.h)
+    __device__ int32_t* misc() const { return S.live - 1; }
+    __device__ int32_t* numLevels() const { return misc() + 3; }  // projection levels of the pool
+    __device__ int32_t* partial() const { return misc() + 4; }    // scan partials, one per warp
+    __device__ int32_t* touching() const { return misc() + 14; }  // a self-contact pair touches this substep
+    __device__ int32_t* numPairs() const { return misc() + 15; }  // how many do
+    // behind the rod's hash in global memory (DRod::hashOff)
+    __device__ int32_t* cursor() const { return S.cellStart + (table + 1); }  // placement cursors
+    __device__ int32_t* lvlOrder() const { return cursor() + (table + 1); }   // coloured mode only
+    __device__ int32_t* lvlStart() const { return lvlOrder() + (selfCapacity + 1); }
+    __device__ int32_t* lvlOf() const { return lvlStart() + (selfCapacity + 1); }
+};
 
 // segCount[j] (zeroed by the caller) += the reference's count of segment j;
-// every touching pair (j, k) is also appended to pairList as (j << 16) | k
-// (*numPairs, zeroed by the caller, counts them; entries past nSt are not
+// every touching pair (j, k) is also appended to S.segStart as (j << 16) | k
+// (*C.numPairs(), zeroed by the caller, counts them; entries past nSt are not
 // stored).
 // Warp w of the team takes chain blocks J = w, w + warps, ...; its lanes test
 // 32 blocks K >= J at a time against J by box distance, and for each block
@@ -146,28 +180,30 @@ __device__ __forceinline__ int bucketMultiplicity(float4 cj, float4 ck, float ce
 // list (which holds nSt pairs; beyond that the count alone is kept and the
 // pool is built from the hash). Not inlined: few pairs get here, and its
 // body is shared by every caller.
-__device__ __noinline__ void countTouching(const RodView& V, const SelfScratch& S, int j, int k, float4 cj,
-                                           float4 ck, float twoR, float cell, int table, int nSt,
-                                           int32_t* touching, int32_t* pairList, int32_t* numPairs) {
+__device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float cell) {
+    const RodView& V = C.V;
+    const SelfScratch& S = C.S;
     const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                        v3(V.x[V.g->sP1[k]]), twoR);
+                                        v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
     if (P.separation >= 0.0f) return;
-    const int mult = bucketMultiplicity(cj, ck, cell, table);
-    if (mult) {
-        atomicAdd(&S.segCount[j], mult);
-        *touching = 1;
-        const int at = atomicAdd(numPairs, 1);
-        if (at < nSt) pairList[at] = (j << 16) | k;
+    const unsigned cells = bucketCells(S.centres[j], S.centres[k], cell, C.table);
+    if (cells) {
+        atomicAdd(&S.segCount[j], __popc(cells));
+        *C.touching() = 1;
+        const int at = atomicAdd(C.numPairs(), 1);
+        if (at < C.nSt) {
+            S.segStart[at] = (j << 16) | k;
+            S.sorted[at] = int32_t(cells);  // for the pool; the hash path rebuilds it
+        }
     }
 }
 
-__device__ void countSelfByBlocks(const RodView& V, const SelfScratch& S, int nSt, int gap, int table,
-                                  float cell, int lane, int team, int32_t* touching, int32_t* pairList,
-                                  int32_t* numPairs) {
+__device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfScratch& S, int nSt, int gap,
+                                                  float radius, float cell, int lane, int team) {
     if (nSt <= gap) return;
     const int wl = lane & 31, warp = lane >> 5, warps = team >> 5;
     const int nBlk = (nSt + 7) >> 3;
-    const float twoR = 2.0f * V.radius;
+    const float twoR = 2.0f * radius;
     // This lane's pair of the block with itself, for the near pairs: the 28
     // pairs (a, b), a < b, of a block ordered by b - a descending, so the
     // pairs with b - a >= gap are a prefix (28 of them for gap 1, 15 for 3).
@@ -198,7 +234,7 @@ __device__ void countSelfByBlocks(const RodView& V, const SelfScratch& S, int nS
             const float bound = pcj.w + ck.w + twoR;
             const float plim = bound * 1.001f + pslack;
             if (ddx * ddx + ddy * ddy + ddz * ddz > plim * plim) return;
-            countTouching(V, S, pj, pk, pcj, ck, twoR, cell, table, nSt, touching, pairList, numPairs);
+            countTouching(C, pj, pk, cell);
         };
         // Near pairs, with no box test (the boxes of J and J + 1 always
         // meet): J against J + 1 in two rounds of 32, J against itself in one
@@ -241,36 +277,6 @@ __device__ void countSelfByBlocks(const RodView& V, const SelfScratch& S, int nS
     }
 }
 
-// What a team needs about its rod beyond its shared-memory arrays: the fixed
-// global pointers, the colour tables, the drive, the self-contact scratch.
-// Lane 0 writes it once per rod into shared memory and every phase reads the
-// fields it uses, so the substep loop carries only the current phase's values
-// in registers (held in registers, these 64-bit pointers filled a third of
-// the register file and pushed the constraint arithmetic into spills). The
-// arrays in shared memory are not reached through it: pointers read back
-// from memory lose their address space, and every access through them
-// would be a generic load.
-struct TeamCtx {
-    RodGlobals G;                   // the rod's fixed global pointers (V.g)
-    RodView V;                      // copies of the view and scratch for the
-    SelfScratch S;                  // separately compiled paths
-    int32_t* cursor;                // hash placement cursors (table entries)
-    int32_t* partial;               // scan partials, one per warp
-    int32_t* numLevels;             // projection levels of the pool
-    int32_t* lvlOrder;
-    int32_t* lvlStart;
-    int32_t* lvlOf;
-    const int* sOrder;
-    const int* bOrder;
-    const int* sCol;
-    const int* bCol;
-    DDrive drive;
-    double tRod;                    // the rod's simulated time (lane 0 advances it)
-    int32_t driveP, wayP, wayStep;  // driven particle, waypoint particle and step
-    int32_t stageFailed;            // a lane gave up waiting for the staged state
-    uint64_t bar;                   // mbarrier of the rod's bulk stage-in
-};
-
 // Polls of the stage-in barrier before a lane gives up (each poll may wait a
 // while in hardware): far beyond any real copy, so it ends only a broken one.
 constexpr int kStageTries = 1 << 20;
@@ -280,45 +286,140 @@ constexpr int32_t kErrorStage = 2;
 // One context per team: a 256-thread CTA holds at most eight one-warp teams.
 constexpr int kMaxTeamsPerCta = 8;
 
-// The projection levels (or colours) of a filled pool of `live` entries, by
-// one thread. S.cellOf serves as the per-particle scratch and must be zero
-// at every particle of the pool.
-__device__ void buildPoolLevels(const TeamCtx& C, int nP, int live, int precision, int32_t* errorWord) {
+// The order in which a filled pool is projected, by the team's first warp:
+// levels such that contacts of one level share no particle and every earlier
+// contact a contact shares a particle with lies in a lower level (level = 1 +
+// the highest among those), so that projecting level by level computes what
+// the serial pool order computes. S.segCount receives each contact's place in
+// level-major order, then the end of every level; *C.numLevels() the count.
+//
+// Bound: the chain of levels through a chunk of 32 contacts, one shuffle per
+// contact that a later one of the chunk depends on. Conflicts inside a chunk
+// come from a mask of its lanes per particle, conflicts with earlier chunks
+// from each particle's last level, both in the shared memory of the count's
+// centres. The serial form, one thread over contacts in global memory, took
+// 35 % of the step of 32 settled rods of 1500-2200 segments (474 contacts in
+// 55 levels).
+//
+// An entry that indexes outside the rod or was left unwritten cuts the pool
+// before it and is reported; it is never dereferenced.
+__device__ __noinline__ void orderPool(const TeamCtx& C, int live, int precision, int32_t* errorWord, int lane) {
+    constexpr unsigned kAll = 0xffffffffu;
     const SelfScratch& S = C.S;
+    const int nP = C.nP;
+    int32_t* const last = reinterpret_cast<int32_t*>(S.centres);   // per particle: its highest level + 1
+    int32_t* const lanes = last + nP;                              // per particle: this chunk's lanes
+    int32_t* const place = S.segCount;
     int kept = live;
-    int n = buildProjectionLevels(S.pool, live, nP, S.cellOf, C.lvlOf, C.lvlOrder, C.lvlStart, &kept);
-    if (precision & kPrecisionColoredSelf) {
-        // colours instead of levels (the valid prefix is known now)
-        for (int i = 0; i < nP; ++i) S.cellOf[i] = 0;
-        const int nc = buildProjectionColors(S.pool, kept, S.cellOf, C.lvlOf, C.lvlOrder, C.lvlStart);
-        if (nc >= 0) {
-            n = nc;
-        } else {  // more than 32 colours: keep the levels
-            for (int i = 0; i < nP; ++i) S.cellOf[i] = 0;
-            n = buildProjectionLevels(S.pool, kept, nP, S.cellOf, C.lvlOf, C.lvlOrder, C.lvlStart, &kept);
+    for (int c0 = 0; c0 < live; c0 += 32) {
+        const int c = c0 + lane;
+        bool ok = true;
+        if (c < live) {
+            const int4 at = *reinterpret_cast<const int4*>(S.pool[c].idx);
+            ok = min(min(at.x, at.y), min(at.z, at.w)) >= 0 && max(max(at.x, at.y), max(at.z, at.w)) < nP &&
+                 S.pool[c].seg != -1;
+            if (ok) {
+                last[at.x] = last[at.y] = last[at.z] = last[at.w] = 0;
+                lanes[at.x] = lanes[at.y] = lanes[at.z] = lanes[at.w] = 0;
+            }
+        }
+        const unsigned bad = __ballot_sync(kAll, !ok);
+        if (bad) {
+            kept = c0 + __ffs(bad) - 1;
+            break;
         }
     }
-    *C.numLevels = n;
-    if (kept != live) {
-        // an entry indexed outside the rod or left unwritten: keep the
-        // valid prefix and report it, never touch memory with it
+    __syncwarp();
+    if (kept != live && lane == 0) {
         *S.live = kept;
         if (errorWord) atomicOr(errorWord, 1);
     }
+    int32_t* const ends = place + kept;
+    if (precision & kPrecisionColoredSelf) {
+        // greedy colours instead (more than 32 of them: the levels)
+        for (int i = lane; i < nP; i += 32) S.cellOf[i] = 0;
+        __syncwarp();
+        int n = 0;
+        if (lane == 0) n = buildProjectionColors(S.pool, kept, S.cellOf, C.lvlOf(), C.lvlOrder(), C.lvlStart());
+        n = __shfl_sync(kAll, n, 0);
+        __syncwarp();
+        if (n >= 0) {
+            for (int i = lane; i < kept; i += 32) place[C.lvlOrder()[i]] = i;
+            for (int l = lane; l < n; l += 32) ends[l] = C.lvlStart()[l + 1];
+            if (lane == 0) *C.numLevels() = n;
+            return;
+        }
+    }
+    int levels = 0;
+    for (int c0 = 0; c0 < kept; c0 += 32) {
+        const int c = c0 + lane;
+        const bool mine = c < kept;
+        int4 at = make_int4(0, 0, 0, 0);
+        int level = 0;
+        if (mine) {
+            at = *reinterpret_cast<const int4*>(S.pool[c].idx);
+            level = max(max(last[at.x], last[at.y]), max(last[at.z], last[at.w]));
+            atomicOr(&lanes[at.x], 1 << lane);
+            atomicOr(&lanes[at.y], 1 << lane);
+            atomicOr(&lanes[at.z], 1 << lane);
+            atomicOr(&lanes[at.w], 1 << lane);
+        }
+        __syncwarp();
+        unsigned before = 0u;  // the chunk's earlier contacts this one shares a particle with
+        if (mine)
+            before = unsigned(lanes[at.x] | lanes[at.y] | lanes[at.z] | lanes[at.w]) & ((1u << lane) - 1u);
+        for (unsigned need = __reduce_or_sync(kAll, before); need; need &= need - 1u) {
+            const int l = __ffs(need) - 1;
+            const int above = __shfl_sync(kAll, level, l) + 1;
+            if ((before >> l) & 1u) level = max(level, above);
+        }
+        if (mine) {
+            place[c] = level;
+            lanes[at.x] = lanes[at.y] = lanes[at.z] = lanes[at.w] = 0;
+            atomicMax(&last[at.x], level + 1);
+            atomicMax(&last[at.y], level + 1);
+            atomicMax(&last[at.z], level + 1);
+            atomicMax(&last[at.w], level + 1);
+        }
+        levels = max(levels, __reduce_max_sync(kAll, mine ? level + 1 : 0));
+        __syncwarp();
+    }
+    // counts per level, their running sum, and each contact's place: a
+    // level's cursor ends at its last contact
+    for (int l = lane; l < levels; l += 32) ends[l] = 0;
+    __syncwarp();
+    for (int c = lane; c < kept; c += 32) atomicAdd(&ends[place[c]], 1);
+    __syncwarp();
+    int sum = 0;
+    for (int l0 = 0; l0 < levels; l0 += 32) {
+        const int l = l0 + lane;
+        const int n = l < levels ? ends[l] : 0;
+        int inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (l < levels) ends[l] = sum + inc - n;
+        sum += __shfl_sync(kAll, inc, 31);
+    }
+    __syncwarp();
+    for (int c = lane; c < kept; c += 32) place[c] = atomicAdd(&ends[place[c]], 1);
+    if (lane == 0) *C.numLevels() = levels;
 }
 
 // The pool fill of a substep on which some segment pair touches: the
-// reference's hash (a stable counting sort), its fill pass in bucket order,
-// and the projection levels (or colours) of the pool. Not inlined: it runs
-// only on substeps with a touching pair, and inlined its registers would
-// count against every phase of the substep loop.
-__device__ __noinline__ void fillSelfPool(const TeamCtx& C, int nSt, int nP, int table, float cell, int live,
-                                          int selfGap, int selfCapacity, float selfFriction, int precision,
-                                          int32_t* errorWord, int lane, int team, int teamIdx) {
+// reference's hash (a stable counting sort) and its fill pass in bucket order.
+// For pools that the pair list cannot give (more than nSt touching pairs).
+// Not inlined: inlined its registers would count against every phase of the
+// substep loop.
+__device__ __noinline__ void fillSelfPool(const TeamCtx& C, float cell, int live, int lane, int team,
+                                          int teamIdx) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
-    int32_t* const& cursor = C.cursor;
-    int32_t* const& partial = C.partial;
+    const int nSt = C.nSt, table = C.table;
+    int32_t* const cursor = C.cursor();
+    int32_t* const partial = C.partial();
         // ---- fill, in the reference's order: its hash buckets ----
         for (int t = lane; t <= table; t += team) S.cellStart[t] = 0;
         for (int c = lane; c < live; c += team) S.pool[c].seg = -1;
@@ -355,15 +456,8 @@ __device__ __noinline__ void fillSelfPool(const TeamCtx& C, int nSt, int nP, int
         }
         teamSync(team, teamIdx);
         for (int j = lane; j < nSt; j += team)
-            if (S.segCount[j] > 0 && S.segStart[j] < selfCapacity)
-                querySelfSegment<true>(V, S, j, nSt, selfGap, table, selfCapacity,
-                                       selfFriction, true);
-        // every thread is done reading the hash (sorted) before
-        // cellOf and sorted (2 nSt >= nP ints) are reused below
-        teamSync(team, teamIdx);
-        for (int i = lane; i < nP; i += team) S.cellOf[i] = 0;
-        teamSync(team, teamIdx);
-        if (lane == 0) buildPoolLevels(C, nP, live, precision, errorWord);
+            if (S.segCount[j] > 0 && S.segStart[j] < C.selfCapacity)
+                querySelfSegment<true>(V, S, j, nSt, C.selfGap, table, C.selfCapacity, C.selfFriction, true);
 }
 
 // Most touching substeps have a handful of touching pairs; for those the
@@ -378,11 +472,9 @@ __device__ __noinline__ void fillSelfPool(const TeamCtx& C, int nSt, int nP, int
 // entry writer: the same pool, entry for entry. Lanes past the capacity
 // write nothing, as the query does. Every lane of the warp calls this; it
 // returns the reference's count of entries. The pair list is
-// S.segStart[0..numPairs), numPairs <= 32; S.segCount holds the pairs' cell
-// masks afterwards, and S.cellOf is zeroed at the pool's particles for the
-// level build.
-__device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int table, float cell,
-                                          int selfCapacity, float selfFriction, int lane) {
+// S.segStart[0..numPairs), numPairs <= 32, with the cells in S.sorted; S.segCount
+// holds the pairs' cells afterwards.
+__device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int lane) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const bool mine = lane < numPairs;
@@ -392,20 +484,15 @@ __device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int ta
         const int pr = S.segStart[lane];
         j = pr >> 16;
         k = pr & 0xffff;
-        cells = bucketCells(S.centres[j], S.centres[k], cell, table);
+        cells = unsigned(S.sorted[lane]);
     }
     const int total = __reduce_add_sync(0xffffffffu, __popc(cells));
     __syncwarp();
     if (mine) S.segCount[lane] = int32_t(cells);
     __syncwarp();
     if (mine) {
-        const int p0 = V.g->sP0[j], p1 = V.g->sP1[j], p2 = V.g->sP0[k], p3 = V.g->sP1[k];
-        S.cellOf[p0] = 0;
-        S.cellOf[p1] = 0;
-        S.cellOf[p2] = 0;
-        S.cellOf[p3] = 0;
-        const SegPair P = segmentPairNarrow(v3(V.x[p0]), v3(V.x[p1]), v3(V.x[p2]), v3(V.x[p3]),
-                                            2.0f * V.radius);
+        const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
+                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
         // entries of the pairs of earlier segments
         int before = 0;
         for (int q = 0; q < numPairs; ++q)
@@ -420,24 +507,138 @@ __device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int ta
                 const unsigned cq = unsigned(S.segCount[q]);
                 rank += __popc(cq & below) + (((cq >> t) & 1u) && (pq & 0xffff) < k ? 1 : 0);
             }
-            if (rank < selfCapacity) writeSelfEntry(V, S.pool[rank], j, k, P, selfFriction);
+            if (rank < C.selfCapacity) writeSelfEntry(V, S.pool[rank], j, k, P, C.selfFriction);
         }
     }
     return total;
 }
 
+// The same pool from any number of listed pairs (at most nSt), by the whole
+// team. Where a segment's entries start is the running sum of the counts;
+// their order within the segment comes from the segment's own pairs, linked
+// per segment (the order of a list is of no matter: ranks are sums over it).
+// Lists and cells lie in the shared memory of the count's centres.
+//
+// Against the hash (build, placement by one warp, and the 27-cell query of
+// every touching segment by one thread each), which bound the step of settled
+// rods: with orderPool above and projectSelfCompact below, 32 settled rods of
+// 1500-2200 segments at 20 substeps 32.4 -> 10.5 ms, 256 of 16-512 at 50
+// substeps 8.53 -> 2.08 ms, and rods in free fall, which touch now and then,
+// 4096 of 16-512, 7.65 -> 6.93 ms.
+__device__ __noinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, int lane, int team, int teamIdx) {
+    const RodView& V = C.V;
+    const SelfScratch& S = C.S;
+    const int nSt = C.nSt;
+    int32_t* const head = reinterpret_cast<int32_t*>(S.centres);  // per segment: its last linked pair
+    int32_t* const next = head + nSt;                             // per pair
+    int32_t* const cellsOf = next + nSt;                          // per pair
+    for (int p = lane; p < numPairs; p += team) {
+        head[S.segStart[p] >> 16] = -1;
+        cellsOf[p] = S.sorted[p];
+    }
+    const int total = teamExclusiveScan(S.segCount, nSt, lane, team, teamIdx, C.partial());
+    for (int p = lane; p < numPairs; p += team) next[p] = atomicExch(&head[S.segStart[p] >> 16], p);
+    teamSync(team, teamIdx);
+    for (int p = lane; p < numPairs; p += team) {
+        const int pr = S.segStart[p], j = pr >> 16, k = pr & 0xffff;
+        const int before = S.segCount[j];
+        if (before >= C.selfCapacity) continue;
+        const unsigned cells = unsigned(cellsOf[p]);
+        const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
+                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
+        for (unsigned rest = cells; rest; rest &= rest - 1u) {
+            const int t = __ffs(rest) - 1;
+            const unsigned below = (1u << t) - 1u;
+            int rank = before;
+            for (int q = head[j]; q >= 0; q = next[q]) {
+                const unsigned cq = unsigned(cellsOf[q]);
+                rank += __popc(cq & below) + (((cq >> t) & 1u) && (S.segStart[q] & 0xffff) < k ? 1 : 0);
+            }
+            if (rank < C.selfCapacity) writeSelfEntry(V, S.pool[rank], j, k, P, C.selfFriction);
+        }
+    }
+    return total;
+}
+
+// Contact c of the pool into its place of the compact, level-major rows in
+// shared memory: {particles}, {u, w}, {n.x, n.y}, {n.z, offset}, {lambdaN,
+// applied}, each a row of `live` 8-byte words.
+__device__ __forceinline__ void compactContact(const SelfScratch& S, int c, int live) {
+    const DSelf& k = S.pool[c];
+    float2* const rows = reinterpret_cast<float2*>(S.centres) + S.segCount[c];
+    rows[0] = make_float2(__int_as_float(k.idx[0] | (k.idx[1] << 16)), __int_as_float(k.idx[2] | (k.idx[3] << 16)));
+    rows[live] = make_float2(k.weight[1], -k.weight[3]);
+    rows[2 * live] = make_float2(k.nx, k.ny);
+    rows[3 * live] = make_float2(k.nz, k.offset);
+    rows[4 * live] = make_float2(0.0f, 0.0f);
+}
+
 // The self-contact pool projected level by level: contacts of one level
 // share no particle, and every earlier contact a contact shares a particle
 // with sits in a lower level -- the serial pool order's result, bit for bit.
-// Not inlined, for the same reason as the fill: it runs only while contacts
-// are live.
+// Not inlined: it runs only while contacts are live. Levels are short (nine
+// contacts on average in settled rods) and there are many, so the chain of
+// one contact's loads and arithmetic per level is what it takes: one warp
+// does them without team barriers unless the levels are wider than a warp,
+// from shared memory (`xAt` .. are byte offsets into it).
 template <bool COMP>
-__device__ __noinline__ void projectSelfLevels(const TeamCtx& C, int nl, int lane, int team, int teamIdx) {
-    for (int l = 0; l < nl; ++l) {
-        for (int c = C.lvlStart[l] + lane; c < C.lvlStart[l + 1]; c += team)
-            projectSelf<COMP>(C.V, C.S.pool[C.lvlOrder[c]]);
-        teamSync(team, teamIdx);
+__device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, int live, int lane, int team,
+                                                int teamIdx) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const RodView& V = C.V;
+    const SelfScratch& S = C.S;
+    // the compiler reaches shared memory with shared-memory instructions only
+    // through a pointer derived from the array itself
+    auto shared = [&](const void* p) { return smem + (static_cast<const unsigned char*>(p) - smem); };
+    float4* const x = reinterpret_cast<float4*>(shared(V.x));
+    float4* const xPrev = reinterpret_cast<float4*>(shared(V.xPrev));
+    float4* const xComp = COMP ? reinterpret_cast<float4*>(shared(V.xComp)) : nullptr;
+    float2* const rows = reinterpret_cast<float2*>(shared(S.centres));
+    const int32_t* const ends = reinterpret_cast<const int32_t*>(shared(S.segCount)) + live;
+    const float friction = C.selfFriction * V.frictionScale;
+    const bool oneWarp = live <= 32 * levels;
+    const int stride = oneWarp ? 32 : team;
+    if (lane < stride) {
+        for (int l = 0, begin = 0; l < levels; ++l) {
+            const int end = ends[l];
+            for (int c = begin + lane; c < end; c += stride) {
+                const float2 i = rows[c], uw = rows[live + c], nxy = rows[2 * live + c], nzo = rows[3 * live + c];
+                float2 lam = rows[4 * live + c];
+                const unsigned a = __float_as_uint(i.x), b = __float_as_uint(i.y);
+                const int at[4] = {int(a & 0xffffu), int(a >> 16), int(b & 0xffffu), int(b >> 16)};
+                const float weight[4] = {1.0f - uw.x, uw.x, -(1.0f - uw.y), -uw.y};
+                const float im[4] = {V.g->invMass[at[0]], V.g->invMass[at[1]], V.g->invMass[at[2]],
+                                     V.g->invMass[at[3]]};
+                const V3 n{nxy.x, nxy.y, nzo.x};
+                const bool distinct = at[0] != at[1] && at[0] != at[2] && at[0] != at[3] && at[1] != at[2] &&
+                                      at[1] != at[3] && at[2] != at[3];
+                if (!distinct || !projectSelfDistinct<COMP>(x, xPrev, xComp, at, weight, im, n, nzo.y, friction,
+                                                            lam.x, lam.y)) {
+                    DSelf k;
+                    for (int m = 0; m < 4; ++m) {
+                        k.idx[m] = at[m];
+                        k.weight[m] = weight[m];
+                    }
+                    k.nx = n.x;
+                    k.ny = n.y;
+                    k.nz = n.z;
+                    k.offset = nzo.y;
+                    k.friction = friction;
+                    k.lambdaN = lam.x;
+                    k.applied = lam.y;
+                    projectSelf<COMP>(V, k);
+                    lam = make_float2(k.lambdaN, k.applied);
+                }
+                rows[4 * live + c] = lam;
+            }
+            begin = end;
+            if (oneWarp)
+                __syncwarp();
+            else
+                teamSync(team, teamIdx);
+        }
     }
+    teamSync(team, teamIdx);
 }
 
 template <bool COMP, bool FP64>
@@ -519,12 +720,12 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         C.V = V;  // for the rarely run, separately compiled paths
         G.view = &C.V;
         C.S = S;
-        C.partial = partial;
-        C.numLevels = numLevels;
-        C.cursor = S.cellStart + (R.hashTableSize + 1);
-        C.lvlOrder = C.cursor + (R.hashTableSize + 1);
-        C.lvlStart = C.lvlOrder + (R.selfCapacity + 1);
-        C.lvlOf = C.lvlStart + (R.selfCapacity + 1);
+        C.nP = nP;
+        C.nSt = nSt;
+        C.table = R.hashTableSize;
+        C.selfGap = R.selfGap;
+        C.selfCapacity = R.selfCapacity;
+        C.selfFriction = R.selfFriction;
         C.sOrder = A.tOrder + T.sOrderOff;
         C.bOrder = A.tOrder + T.bOrderOff;
         C.sCol = A.tColorStart + T.sColorOff;
@@ -535,10 +736,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         // one-step-per-launch path advances rodTime[r]
         C.tRod = A.rodTime[r];
         C.driveP = -1;
-        C.drive = DDrive{};
         if (A.drives) {
-            C.drive = A.drives[r];
-            if (C.drive.particle >= 0 && C.drive.particle < nP) C.driveP = C.drive.particle;
+            const int p = A.drives[r].particle;
+            if (p >= 0 && p < nP) C.driveP = p;
         }
         C.wayP = -1;  // waypoint schedule: its particle and step count
         C.wayStep = 0;
@@ -583,12 +783,11 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     const float h = A.h, invH2 = A.invH2;
     const int interval = A.contactInterval;
     const bool self = R.selfCollision != 0;
-    const int table = R.hashTableSize;
 
     const int stepsHere = A.stepsPerLaunch > 0 ? A.stepsPerLaunch : 1;
     for (int step = 0; step < stepsHere; ++step) {
         if (lane == 0) {
-            if (C.driveP >= 0) V.g->kin[C.driveP] = driveVelocityB(C.drive, C.tRod);
+            if (C.driveP >= 0) V.g->kin[C.driveP] = driveVelocityB(A.drives[r], C.tRod);
             if (C.wayP >= 0) V.g->kin[C.wayP] = waypointVelocity(A.waypoints[r], C.wayStep + step);
         }
         teamSync(team, teamIdx);
@@ -697,53 +896,43 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     // ---- count: contacts per segment, by chain blocks ----
                     // chain-block bounds and zeroed counts come from the centre pass
                     // the pair list takes segStart, which the hash path rebuilds
-                    countSelfByBlocks(V, S, nSt, R.selfGap, table, cell, lane, team, touching, S.segStart,
-                                      numPairs);
+                    countSelfByBlocks(C, S, nSt, C.selfGap, V.radius, cell, lane, team);
                     teamSync(team, teamIdx);
                     // team-uniform: shared words read after the barrier
                     const int pairs = *touching ? *numPairs : 0;
-                    if (pairs > 0 && pairs <= 32 && pairs <= nSt) {
-                        int total = 0;
-                        if (lane < 32)
-                            total = poolFromPairs(C, pairs, table, cell, R.selfCapacity, R.selfFriction, lane);
-                        const int live = total < R.selfCapacity ? total : R.selfCapacity;
-                        if (lane == 0) {
-                            *S.live = live;
-                            if (total > R.selfCapacity) *S.overflow += total - R.selfCapacity;
+                    int total = 0;
+                    if (pairs > 0 && pairs <= nSt) {
+                        if (pairs <= 32) {
+                            if (lane < 32)
+                                total = poolFromPairs(C, pairs, lane);
+                        } else {
+                            total = poolFromManyPairs(C, pairs, lane, team, teamIdx);
                         }
+                    } else if (pairs > 0) {
+                        for (int j = lane; j < nSt; j += team) S.segStart[j] = S.segCount[j];
+                        teamSync(team, teamIdx);
+                        total = teamExclusiveScan(S.segStart, nSt, lane, team, teamIdx, partial);
+                        fillSelfPool(C, cell, min(total, C.selfCapacity), lane, team, teamIdx);
+                    }
+                    if (lane == 0) {
+                        *S.live = min(total, C.selfCapacity);
+                        if (total > C.selfCapacity) *S.overflow += total - C.selfCapacity;
+                        if (pairs == 0) *numLevels = 0;
+                    }
+                    if (pairs > 0) {  // team-uniform
                         teamSync(team, teamIdx);  // pool written, positions read: the prediction may start
-                        if (lane == 0)
-                            buildPoolLevels(C, nP, live, A.precision, A.errors ? A.errors + r : nullptr);
-                    } else {
-                        int total = 0;
-                        if (pairs > 0) {
-                            for (int j = lane; j < nSt; j += team) S.segStart[j] = S.segCount[j];
-                            teamSync(team, teamIdx);
-                            total = teamExclusiveScan(S.segStart, nSt, lane, team, teamIdx, partial);
-                        }
-                        const int live = total < R.selfCapacity ? total : R.selfCapacity;
-                        if (lane == 0) {
-                            *S.live = live;
-                            if (total > R.selfCapacity) *S.overflow += total - R.selfCapacity;
-                        }
-                        if (live > 0) {
-                            fillSelfPool(C, nSt, nP, table, cell, live, R.selfGap, R.selfCapacity, R.selfFriction,
-                                         A.precision, A.errors ? A.errors + r : nullptr, lane, team, teamIdx);
-                        } else if (lane == 0) {
-                            *numLevels = 0;
-                        }
+                        if (lane < 32)
+                            orderPool(C, *S.live, A.precision, A.errors ? A.errors + r : nullptr, lane);
                     }
-                } else if (lane == 0) {
-                    for (int c = 0; c < *S.live; ++c) {
-                        S.pool[c].lambdaN = 0.0f;
-                        S.pool[c].applied = 0.0f;
-                    }
+                } else {
+                    float2* const lam = reinterpret_cast<float2*>(S.centres) + 4 * *S.live;
+                    for (int c = lane; c < *S.live; c += team) lam[c] = make_float2(0.0f, 0.0f);
                 }
                 // no barrier here: every read of positions above finished before
                 // an earlier barrier, the prediction below touches neither the
-                // pool nor the level tables, and what lane 0 writes last (live
-                // count, levels) is read only after the prediction's barrier --
-                // so the team predicts while lane 0 builds the levels
+                // pool nor its order, and what the first warp writes last
+                // is read only after the prediction's barrier -- so the other
+                // warps predict while it orders the pool
             }
             // the previous substep's velocity update runs here, fused with this
             // substep's prediction: nothing between them reads v or omega,
@@ -760,6 +949,10 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 predictFrameFrom<COMP>(V, j, h, wj, nullptr);
             }
             teamSync(team, teamIdx);
+            // the ordered pool into shared memory, read again only after the
+            // barriers of the sweeps below
+            if (self && regenerate && *numLevels > 0)
+                for (int c = lane; c < *S.live; c += team) compactContact(S, c, *S.live);
 
             for (int it = 0; it < A.iterations; ++it) {
                 // a chain coloured even/odd: constraint k of colour c is
@@ -811,11 +1004,8 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     teamSync(team, teamIdx);
                 }
                 if (self) {
-                    // level by level: contacts of one level share no particle, and
-                    // every earlier contact a contact shares a particle with sits in
-                    // a lower level -- the serial pool order's result, bit for bit
                     const int nl = *numLevels;
-                    if (nl > 0) projectSelfLevels<COMP>(C, nl, lane, team, teamIdx);
+                    if (nl > 0) projectSelfCompact<COMP>(C, nl, *S.live, lane, team, teamIdx);
                 }
             }
 

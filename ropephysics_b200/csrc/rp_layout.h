@@ -30,8 +30,12 @@
 //   misc       kMiscBytes (below)
 //   self       full: centres 16 nSt, ints 16 nSt, hash 4 (table + 1) x 2,
 //              pool 64 x capacity, projection levels 3 x 4 (capacity + 1);
-//              lean: centres 16 nSt, count and start 8 nSt, chain-block
-//              bounds 32 x ceil(nSt / 8) (the rest in global memory)
+//              lean: centres 16 nSt, chain-block bounds 32 x ceil(nSt / 8),
+//              count and start 8 nSt (the rest in global memory). The count
+//              is done with all of them when the pool stands, so the first
+//              two then hold its contacts, in projection order, and the last
+//              the order (kCompactBytes and 8 bytes a contact: short rods
+//              are rounded up to their 16 contacts)
 #pragma once
 
 #include <cstdint>
@@ -60,6 +64,11 @@ struct RodLayout {
 //   [15] touching pairs found by the count (batched)
 //   [16..79] per-warp reduction rows (8 warps x 8 floats)
 constexpr int32_t kMiscBytes = 320;
+
+// Shared memory of one self contact while it is projected (batched kernel):
+// five 8-byte rows. A pool of nSt / 2 of them is the 20 nSt bytes that the
+// count's centres and block bounds take.
+constexpr int32_t kCompactBytes = 40;
 
 RP_HD inline int32_t rpAlign16(int32_t b) { return (b + 15) & ~15; }
 
@@ -122,10 +131,13 @@ RP_HD inline RodLayout rodLayout(int32_t nP, int32_t nS, int32_t nSt, int32_t nB
         // lean: what the count reads every substep; the hash, the sort and
         // the projection levels (touched only while a pair touches) and the
         // pool live in global memory
-        L.centres = o; o += 16 * nSt;
-        L.selfInt = o; o += rpAlign16(8 * nSt);  // per-segment count and start
+        const int32_t most = 32 * kCompactBytes / 2;  // the smallest pool, 16 contacts
+        const int32_t count = 16 * nSt + 32 * ((nSt + 7) / 8);
+        L.centres = o;
+        L.blocks = o + 16 * nSt;
+        o += count > most ? count : most;
+        L.selfInt = o; o += nSt > 16 ? rpAlign16(8 * nSt) : 128;  // per-segment count and start
         L.hash = L.pool = L.levels = -1;
-        L.blocks = o;  o += 32 * ((nSt + 7) / 8);
     } else {
         L.centres = L.selfInt = L.hash = L.pool = L.levels = o;
         L.blocks = -1;

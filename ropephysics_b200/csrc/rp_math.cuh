@@ -109,8 +109,8 @@ __device__ __forceinline__ V3 cwise(V3 a, V3 b) { return V3{a.x * b.x, a.y * b.y
 // 2^-149 away. Outside the ranges -- NaN, infinities, singular matrices --
 // `ok` turns false and the caller falls back to the plain operators. Signs
 // of zero are kept too (b > 0).
-constexpr float kRootLo = 0x1p-64f, kRootHi = 0x1p64f;  // operands of sqrtRecip
-constexpr float kDivLo = 0x1p-32f, kDivHi = 0x1p32f;    // divisors
+constexpr float kRootLo = 0x1p-100f, kRootHi = 0x1p100f;  // operands of sqrtRecip
+constexpr float kDivLo = 0x1p-62f, kDivHi = 0x1p62f;      // divisors
 
 // A divisor b > 0 and its reciprocal y = RN(1 / b), with the scaled pair that
 // the residual uses.

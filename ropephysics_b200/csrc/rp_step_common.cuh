@@ -660,49 +660,6 @@ __device__ __forceinline__ void querySelfSegment(const RodView& V, const SelfScr
     if (!fill) S.segCount[j] = count;
 }
 
-// Levels for projecting a self-contact pool in parallel with the serial
-// pool order's result: level(c) = 1 + the highest level among earlier
-// contacts that share a particle with c. Contacts of one level touch disjoint
-// particles, and every earlier contact that c depends on sits in a lower
-// level, so projecting level by level computes exactly what the serial loop
-// computes. `last` holds one zeroed int per particle; `lvlOf` one int per
-// contact. Fills order[live] (contacts grouped by level, pool order within a
-// level) and start[levels + 1]; returns the number of levels. Entries whose
-// particle indices fall outside [0, nP), or marked unwritten (seg == -1), are
-// never dereferenced: the pool is cut before the first of them and *kept says
-// how many entries remain. One thread.
-__device__ __forceinline__ int buildProjectionLevels(const DSelf* pool, int live, int nP, int32_t* last,
-                                                     int32_t* lvlOf, int32_t* order, int32_t* start,
-                                                     int* kept) {
-    for (int c = 0; c < live; ++c) {
-        const DSelf& k = pool[c];
-        bool ok = true;
-        for (int m = 0; m < 4; ++m) ok = ok && k.idx[m] >= 0 && k.idx[m] < nP;
-        ok = ok && k.seg != -1;  // -1: a slot the filling pass left unwritten
-        if (!ok) {
-            live = c;
-            break;
-        }
-    }
-    *kept = live;
-    int levels = 0;
-    for (int c = 0; c < live; ++c) {
-        const DSelf& k = pool[c];
-        int l = 0;
-        for (int m = 0; m < 4; ++m) l = max(l, last[k.idx[m]]);
-        lvlOf[c] = l;
-        for (int m = 0; m < 4; ++m) last[k.idx[m]] = l + 1;
-        levels = max(levels, l + 1);
-    }
-    for (int l = 0; l <= levels; ++l) start[l] = 0;
-    for (int c = 0; c < live; ++c) ++start[lvlOf[c] + 1];
-    for (int l = 0; l < levels; ++l) start[l + 1] += start[l];
-    for (int c = 0; c < live; ++c) order[start[lvlOf[c]]++] = c;
-    for (int l = levels; l > 0; --l) start[l] = start[l - 1];
-    start[0] = 0;
-    return levels;
-}
-
 // Greedy colours for projecting a self-contact pool in parallel (the
 // reference's proposed speed-up for its serial self-contact loop,
 // REMAINING.md:14-17): in pool order, each contact takes the lowest colour
@@ -710,11 +667,12 @@ __device__ __forceinline__ int buildProjectionLevels(const DSelf* pool, int live
 // disjoint particles, so a colour projects in parallel exactly as in any
 // order; the colours run in ascending order. This is a different
 // Gauss-Seidel order from the serial loop's, so results differ from it (the
-// levels above reproduce it). `used` holds one zeroed int per particle (a
-// bitmask of its colours), `colOf` one int per contact; fills order/start as
-// buildProjectionLevels does and returns the number of colours, or -1 when a
-// contact would need a 33rd colour (`used` is then dirty). The first `live`
-// entries must be valid (buildProjectionLevels' prefix check). One thread.
+// batched kernel's levels reproduce it). `used` holds one zeroed int per
+// particle (a bitmask of its colours), `colOf` one int per contact; fills
+// order[live] (contacts grouped by colour, pool order within a colour) and
+// start[colours + 1] and returns the number of colours, or -1 when a
+// contact would need a 33rd colour. The first `live` entries must be valid
+// (written, and indexing inside the rod). One thread.
 __device__ __forceinline__ int buildProjectionColors(const DSelf* pool, int live, int32_t* used,
                                                      int32_t* colOf, int32_t* order, int32_t* start) {
     int colors = 0;
@@ -735,6 +693,94 @@ __device__ __forceinline__ int buildProjectionColors(const DSelf* pool, int live
     for (int l = colors; l > 0; --l) start[l] = start[l - 1];
     start[0] = 0;
     return colors;
+}
+
+// The four-particle case of the contact projection on distinct particles,
+// with everything read before anything is written: the reads of positions,
+// displacements and masses overlap, where projectSelf waits for each
+// particle's store before it reads the next. `lambdaN` and `applied` are the
+// contact's multipliers, updated in place. Returns false, having written
+// nothing, for what the shared reciprocals do not cover (projectSelf does it).
+template <bool COMP>
+__device__ __forceinline__ bool projectSelfDistinct(float4* x, float4* xPrev, float4* xComp, const int (&at)[4],
+                                                    const float (&weight)[4], const float (&im)[4], V3 n,
+                                                    float offset, float friction, float& lambdaN,
+                                                    float& applied) {
+    float wEff = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) wEff = fma3(weight[m] * weight[m], im[m], wEff);
+    if (wEff <= 0.0f) return true;
+    bool ok = true;
+    const Divisor dw = divisor(wEff, recip(wEff, ok));
+    ok = ok & (fmaxf(fmaxf(im[0], im[1]), fmaxf(im[2], im[3])) <= 0x1p60f);
+    V3 p[4], c[4], d[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        p[m] = v3(x[at[m]]);
+        d[m] = v3(xPrev[at[m]]);
+        if (COMP) c[m] = v3(xComp[at[m]]);
+    }
+    // addPos on the values held here
+    auto add = [&](int m, V3 a, float s) {
+        if (!COMP) {
+            p[m] = fmav(a, s, p[m]);
+        } else {
+            const V3 step = a * s;
+            const V3 y = step - c[m];
+            const V3 t = p[m] + y;
+            c[m] = (t - p[m]) - y;
+            p[m] = t;
+            d[m] = d[m] + step;
+        }
+    };
+    float C = -offset;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) C = fma3(weight[m], dot(p[m], n), C);
+    float dLambda = quotient(-C, dw);
+    ok = ok & (fabsf(dLambda) <= 0x1p60f);
+    const float clamped = lambdaN + dLambda > 0.0f ? lambdaN + dLambda : 0.0f;
+    dLambda = clamped - lambdaN;
+    const float lambda = clamped;
+    float rubbed = applied;
+    if (dLambda != 0.0f) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) add(m, n, im[m] * weight[m] * dLambda);
+    }
+    if (!(friction <= 0.0f || lambda <= 0.0f)) {
+        V3 dp{0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) dp = fmav(COMP ? d[m] : p[m] - d[m], weight[m], dp);
+        const V3 tangential = fmav(-n, dot(dp, n), dp);  // dp - n (dp . n)
+        const float slide2 = norm2(tangential);
+        // below 1e-15 (its square under 2^-99) nothing slides, and projectSelf
+        // returns as well
+        if (slide2 >= kRootLo) {
+            float slide, invSlide;
+            sqrtRecip(slide2, slide, invSlide, ok);
+            const float budget = fma3(friction * lambda, wEff, -rubbed);
+            if (!(slide < 1e-15f || budget <= 0.0f)) {
+                const float capped = slide < budget ? slide : budget;
+                rubbed += capped;
+                const V3 correction = tangential * quotient(-capped, divisor(slide, invSlide));
+#pragma unroll
+                for (int m = 0; m < 4; ++m) add(m, correction, quotient(im[m] * weight[m], dw));
+            }
+        } else {
+            ok = ok & (slide2 < kRootLo);  // not NaN
+        }
+    }
+    if (!ok) return false;
+    lambdaN = lambda;
+    applied = rubbed;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        x[at[m]] = f4(p[m]);
+        if (COMP) {
+            xComp[at[m]] = f4(c[m]);
+            xPrev[at[m]] = f4(d[m]);
+        }
+    }
+    return true;
 }
 
 // The four-particle case of the contact projection.

@@ -130,9 +130,9 @@ int main() {
 """
 
 # how many inputs each comparison must have covered: the floats of
-# [2^-64, 2^64], of [2^-32, 2^32], the near-boundary quotients, and most of
+# [2^-100, 2^100], of [2^-62, 2^62], the near-boundary quotients, and most of
 # the random solves
-COVERED = [128 * (1 << 23), 64 * (1 << 23), 200_000_000, 592 * 256 * 4096 // 2]
+COVERED = [200 * (1 << 23), 124 * (1 << 23), 200_000_000, 592 * 256 * 4096 // 2]
 
 
 @pytest.mark.gpu
