@@ -378,51 +378,13 @@ namespace rpx {
 rp_status buildBatchedPlan(rp_batch* b, const Tune& tune, int precision) {
     // Length-sorted work order: longest first, so the tail of the persistent
     // queue is short rods and the SMs finish together.
-    std::vector<int32_t> ids(b->numRods), order, groups;
+    std::vector<int32_t> ids(b->numRods);
     for (int r = 0; r < b->numRods; ++r) ids[r] = r;
-    const int cta = tune.ctaThreads;
-    const bool comp = (precision & RP_PRECISION_COMPENSATED) != 0;
-    const size_t optin = optinSmem(b->device);
-    const size_t fixed = rp::batchedStaticSmem() + 64;  // the kernel's own shared memory
-    // World contact slots go into shared memory when the groups still fit as
-    // many CTAs per SM with them (few contact primitives per rod, or short
-    // rods); otherwise they stay in global memory.
-    size_t maxSmem = rpx::planGroups(ids, b->rods.data(), b->tmpls.data(), cta, tune.pairsPerThread, comp,
-                                     order, groups, false);
-    if (maxSmem == rpx::kMisaligned)
-        return fail(RP_ERR_INVALID, "internal: a rod's shared-memory layout is not 16-byte aligned");
-    int slotsShared = 0;
-    if (b->maxPrims > 0) {
-        std::vector<int32_t> order2, groups2;
-        const size_t smem2 = rpx::planGroups(ids, b->rods.data(), b->tmpls.data(), cta, tune.pairsPerThread,
-                                             comp, order2, groups2, true);
-        int per1 = 0, per2 = 0;
-        if (smem2 != rpx::kMisaligned && smem2 + fixed <= optin &&
-            rp::batchedReserveSmem(std::max(smem2, maxSmem)) == cudaSuccess &&
-            rp::batchedOccupancy(cta, maxSmem, precision, &per1) == cudaSuccess &&
-            rp::batchedOccupancy(cta, smem2, precision, &per2) == cudaSuccess && per2 >= per1 && per2 >= 1) {
-            maxSmem = smem2;
-            order.swap(order2);
-            groups.swap(groups2);
-            slotsShared = 1;
-        }
-        cudaGetLastError();
-    }
-    if (maxSmem + fixed > optin)
-        return fail(RP_ERR_SHARED_MEMORY, "a rod group needs " + std::to_string(maxSmem) +
-                                              " bytes of shared memory; the device allows " +
-                                              std::to_string(optin));
-    if (rp::batchedReserveSmem(std::max<size_t>(maxSmem, 1)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(RP_ERR_SHARED_MEMORY, "cannot opt into the batched shared memory");
-    }
-    int perSm = 0;
-    if (rp::batchedOccupancy(cta, maxSmem, precision, &perSm) != cudaSuccess || perSm < 1) {
-        cudaGetLastError();
-        return fail(RP_ERR_SHARED_MEMORY, "batched kernel cannot be resident with this group size");
-    }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    rpx::BatchedShape shape;
+    const rp_status planned = rpx::planBatched(ids, b->rods.data(), b->tmpls.data(), tune.ctaThreads,
+                                               tune.pairsPerThread, precision, b->device, b->maxPrims > 0, shape);
+    if (planned != RP_OK) return planned;
+    std::vector<int32_t>&order = shape.order, &groups = shape.groups;
     const int numGroups = int(groups.size() / 4);
     rp_status st;
     if (!b->dQueue && (st = b->alloc(b->dQueue, 2)) != RP_OK) return st;
@@ -467,11 +429,11 @@ rp_status buildBatchedPlan(rp_batch* b, const Tune& tune, int precision) {
     b->owned.push_back(newGroups);
     b->groups.swap(groups);
     b->numGroups = numGroups;
-    b->a.slotsShared = slotsShared;
+    b->a.slotsShared = shape.slotsShared;
     b->a.work = b->dWork;
-    b->batchedSmem = maxSmem;
-    b->batchedThreads = cta;
-    b->batchedBlocks = std::max(1, std::min(numGroups, sms * perSm));
+    b->batchedSmem = shape.smem;
+    b->batchedThreads = shape.cta;
+    b->batchedBlocks = shape.blocks;
     b->tune.ctaThreads = tune.ctaThreads;
     b->tune.pairsPerThread = tune.pairsPerThread;
     return RP_OK;

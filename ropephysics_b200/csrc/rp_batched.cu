@@ -4,7 +4,8 @@
 // (longest first). A group is up to CTA/team rods that share a team size; the
 // team size grows with the rod (about one thread per two segments, whole
 // warps, 32..256), so a 64-segment rod is one warp and a 512-segment rod is
-// eight. A persistent grid sized to the SMs' resident capacity pulls groups
+// eight; launches that leave half the GPU idle get about one thread per
+// segment, up to 512 (planBatched). A persistent grid sized to the SMs' resident capacity pulls groups
 // from a global counter, so long and short rods mix freely across SMs and the
 // tail of the queue is short work.
 //
@@ -153,7 +154,7 @@ struct TeamCtx {
     // the rod's misc words (rp_layout.h)
     __device__ int32_t* misc() const { return S.live - 1; }
     __device__ int32_t* numLevels() const { return misc() + 3; }  // projection levels of the pool
-    __device__ int32_t* partial() const { return misc() + 4; }    // scan partials, one per warp
+    __device__ int32_t* partial() const { return misc() + 16; }   // scan partials, one per warp
     __device__ int32_t* touching() const { return misc() + 14; }  // a self-contact pair touches this substep
     __device__ int32_t* numPairs() const { return misc() + 15; }  // how many do
     // behind the rod's hash in global memory (DRod::hashOff)
@@ -283,7 +284,7 @@ constexpr int kStageTries = 1 << 20;
 // DArgs::errors bit of a rod whose state copy never completed
 constexpr int32_t kErrorStage = 2;
 
-// One context per team: a 256-thread CTA holds at most eight one-warp teams.
+// One context per team: a group holds at most eight rods.
 constexpr int kMaxTeamsPerCta = 8;
 
 // The order in which a filled pool is projected, by the team's first warp:
@@ -693,7 +694,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     S.live = misc + 1;
     S.overflow = misc + 2;
     S.blocks = reinterpret_cast<float4*>(base + L.blocks);
-    int32_t* partial = misc + 4;  // one per warp of the team (up to 8)
+    int32_t* partial = misc + 16;  // one per warp of the team
     int32_t* numLevels = misc + 3;
     unsigned long long* primMask = reinterpret_cast<unsigned long long*>(misc + 12);
     int32_t* touching = misc + 14;
@@ -1068,7 +1069,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 }
 
 template <bool COMP, bool FP64>
-__global__ void __launch_bounds__(256, 2) kBatchedStep(DArgs A, const int32_t* __restrict__ groups,
+__global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* __restrict__ groups,
                                                        int numGroups, int32_t* queue) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sGroup;

@@ -51,11 +51,16 @@ struct TemplateHost {
     std::vector<char> fixed;
 };
 void makeTemplate(const rp_rod_desc* d, TemplateHost& out);
-int teamThreads(int nSt, int pairsPerThread);
-constexpr size_t kMisaligned = ~size_t(0);
-size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls,
-                  int cta, int pairsPerThread, bool comp, std::vector<int32_t>& order,
-                  std::vector<int32_t>& groups, bool slotsShared = false);
+// The batched kernel's launch over a set of rods.
+struct BatchedShape {
+    std::vector<int32_t> order, groups;  // rods longest first; four ints per group
+    int cta = 256;                       // threads per CTA
+    int blocks = 1;                      // persistent grid
+    size_t smem = 0;                     // dynamic shared memory per CTA
+    int slotsShared = 0;                 // world contact slots in shared memory
+};
+rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
+                      int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out);
 
 // ---- rp_batch.cpp: what the trajectory writer reads of a batch ----
 struct BatchView {

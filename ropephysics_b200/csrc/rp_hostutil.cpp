@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "rp_host.h"
+#include "rp_launch.h"
 #include "rp_layout.h"
 
 namespace rpx {
@@ -193,7 +194,24 @@ void makeTemplate(const rp_rod_desc* d, TemplateHost& h) {
                      : 0);
 }
 
-int teamThreads(int nSt, int pairsPerThread) {
+namespace {
+
+constexpr size_t kMisaligned = ~size_t(0);
+constexpr int kNoWide = INT32_MAX;
+
+// Threads of a rod's team: about one per two segments (a colour's constraints
+// one to a lane), whole warps, 32..256. A rod longer than `wideFrom` gets about one
+// per segment instead, a power of two, for launches that leave room (see
+// planBatched): up to 512 where a lane still has more than one constraint of a
+// colour or a self-contact count to share, else up to 256 (512 segments without
+// self-collision: 152 us a step with 256 threads, 166 with 512).
+int teamThreads(int nSt, bool self, int pairsPerThread, int wideFrom) {
+    if (nSt > wideFrom) {
+        const int most = self || nSt > 512 ? 512 : 256;
+        int t = 32;
+        while (t < most && 2 * nSt > 3 * t) t *= 2;
+        return t;
+    }
     int t = (nSt / 2 + pairsPerThread - 1) / pairsPerThread;
     t = (t + 31) / 32 * 32;
     return std::max(32, std::min(256, t));
@@ -206,26 +224,28 @@ int teamThreads(int nSt, int pairsPerThread) {
 // `order`, rod count, team size, shared bytes. Returns the largest group's
 // shared bytes.
 size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls,
-                  int cta, int pairsPerThread, bool comp, std::vector<int32_t>& order,
-                  std::vector<int32_t>& groups, bool slotsShared) {
+                  int cta, int pairsPerThread, int wideFrom, bool comp, bool slotsShared,
+                  std::vector<int32_t>& order, std::vector<int32_t>& groups) {
     order = rodIds;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return tmpls[rods[x].tmpl].nSt > tmpls[rods[y].tmpl].nSt;
     });
+    auto teamOf = [&](int r) {
+        return std::min(cta, teamThreads(tmpls[rods[r].tmpl].nSt, rods[r].selfCollision != 0, pairsPerThread, wideFrom));
+    };
     groups.clear();
     size_t maxSmem = 0;
     const int n = int(order.size());
     int i = 0;
     while (i < n) {
-        const rp::DRod& R0 = rods[order[i]];
-        const int team = std::min(cta, teamThreads(tmpls[R0.tmpl].nSt, pairsPerThread));
-        const int perCta = cta / team;
+        const int team = teamOf(order[i]);
+        const int perCta = std::min(8, cta / team);  // the kernel holds eight team contexts
         int cnt = 0;
         size_t smem = 0;
         while (i + cnt < n && cnt < perCta) {
             const rp::DRod& R = rods[order[i + cnt]];
             const rp::DTemplate& T = tmpls[R.tmpl];
-            if (std::min(cta, teamThreads(T.nSt, pairsPerThread)) != team) break;
+            if (teamOf(order[i + cnt]) != team) break;
             const rp::RodLayout L = rp::rodLayout(T.nP, T.nS, T.nSt, T.nB, R.numPrims, R.selfCollision,
                                                   R.hashTableSize, R.selfCapacity, 1, comp ? 1 : 0,
                                                   slotsShared ? 1 : 0);
@@ -241,6 +261,104 @@ size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, cons
         i += cnt;
     }
     return maxSmem;
+}
+
+// One launch shape: its groups, its shared memory, and how many of its CTAs
+// an SM holds.
+rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
+                    int pairsPerThread, int wideFrom, int precision, size_t optin, bool mayShareSlots,
+                    BatchedShape& out, int* perSm) {
+    const bool comp = (precision & RP_PRECISION_COMPENSATED) != 0;
+    const size_t fixed = rp::batchedStaticSmem() + 64;  // the kernel's own shared memory
+    out.cta = cta;
+    out.slotsShared = 0;
+    out.smem = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, false, out.order, out.groups);
+    if (out.smem == kMisaligned)
+        return fail(RP_ERR_INVALID, "internal: a rod's shared-memory layout is not 16-byte aligned");
+    // World contact slots go into shared memory when the groups still fit as
+    // many CTAs per SM with them (few contact primitives per rod, or short
+    // rods); otherwise they stay in global memory.
+    if (mayShareSlots) {
+        std::vector<int32_t> order2, groups2;
+        const size_t smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, order2,
+                                        groups2);
+        int per1 = 0, per2 = 0;
+        if (smem2 != kMisaligned && smem2 + fixed <= optin &&
+            rp::batchedReserveSmem(std::max(smem2, out.smem)) == cudaSuccess &&
+            rp::batchedOccupancy(cta, out.smem, precision, &per1) == cudaSuccess &&
+            rp::batchedOccupancy(cta, smem2, precision, &per2) == cudaSuccess && per2 >= per1 && per2 >= 1) {
+            out.smem = smem2;
+            out.order.swap(order2);
+            out.groups.swap(groups2);
+            out.slotsShared = 1;
+        }
+        cudaGetLastError();
+    }
+    if (out.smem + fixed > optin)
+        return fail(RP_ERR_SHARED_MEMORY, "a rod group needs " + std::to_string(out.smem) +
+                                              " bytes of shared memory; the device allows " +
+                                              std::to_string(optin));
+    if (rp::batchedReserveSmem(std::max<size_t>(out.smem, 1)) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(RP_ERR_SHARED_MEMORY, "cannot opt into the batched shared memory");
+    }
+    if (rp::batchedOccupancy(cta, out.smem, precision, perSm) != cudaSuccess || *perSm < 1) {
+        cudaGetLastError();
+        return fail(RP_ERR_SHARED_MEMORY, "batched kernel cannot be resident with this group size");
+    }
+    return RP_OK;
+}
+
+}  // namespace
+
+// The launch of the batched kernel over `rodIds` with the asked CTA size and
+// segment pairs per thread.
+//
+// The default shape (256 threads, one pair per thread) gives a rod the threads
+// its constraint colours need, which is best while the GPU is full. With fewer
+// rods the step takes as long as its slowest rod, and the phases with one
+// item per segment or more (prediction, contacts, the self-contact count) gain
+// from twice the team. So as many of the longest rods as still leave every group
+// of the launch resident at once, on half the GPU's threads, get about one
+// thread per segment: all of them if that fits, else those longer than 64,
+// 128, ... 448 segments. Beyond half, a batch alone still gains a little, but
+// batches on other streams are kept out of the SMs (three batches of 296 rods of
+// 200, 20 substeps: 93 us a step each against 130).
+//
+// Measured on a B200, 20 substeps, one batch alone (three at once, a step
+// each): one rod of 64 126 -> 118 us (51 -> 44), 64 of 128 148 -> 124 (61 -> 52),
+// 16 of 900 295 -> 222 (112 -> 84), 64 settled rods of 40-200 with
+// self-collision 1271 -> 968 (447 -> 355).
+rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
+                      int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out) {
+    const size_t optin = optinSmem(device);
+    int sms = 0, perSm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (cta == 256 && pairsPerThread == 1) {
+        int longest = 0;
+        for (int32_t r : rodIds) longest = std::max(longest, tmpls[rods[r].tmpl].nSt);
+        for (int wideFrom = 0; wideFrom < std::min(longest, 449); wideFrom += 64) {
+            int64_t threads = 0;
+            int most = 128;
+            for (int32_t r : rodIds) {
+                const int team = teamThreads(tmpls[rods[r].tmpl].nSt, rods[r].selfCollision != 0, 1, wideFrom);
+                threads += team;
+                most = std::max(most, team);
+            }
+            if (threads > int64_t(sms) * 256) continue;
+            const int wideCta = most <= 128 ? 128 : most <= 256 ? 256 : 512;
+            if (planShape(rodIds, rods, tmpls, wideCta, 1, wideFrom, precision, optin, mayShareSlots, out, &perSm) ==
+                    RP_OK &&
+                int(out.groups.size() / 4) <= sms * perSm) {
+                out.blocks = std::max(1, int(out.groups.size() / 4));
+                return RP_OK;
+            }
+        }
+    }
+    const rp_status st = planShape(rodIds, rods, tmpls, cta, pairsPerThread, kNoWide, precision, optin, mayShareSlots,
+                                   out, &perSm);
+    if (st == RP_OK) out.blocks = std::max(1, std::min(int(out.groups.size() / 4), sms * perSm));
+    return st;
 }
 
 }  // namespace rpx

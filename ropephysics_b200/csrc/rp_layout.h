@@ -59,11 +59,14 @@ struct RodLayout {
 
 // Per-rod scalars and team reduction scratch, as 32-bit words:
 //   [0] cell size  [1] live pool entries  [2] overflow  [3] projection levels
-//   [4..11] per-warp scan partials  [12..13] primitive mask (64 bits)
+//   [12..13] primitive mask (64 bits)
 //   [14] a self-contact pair touches this substep (batched)
 //   [15] touching pairs found by the count (batched)
-//   [16..79] per-warp reduction rows (8 warps x 8 floats)
+//   [16..] per-warp reduction rows (8 floats a warp), reused for the per-warp
+//   scan partials: 8 rows; 16 for rods of more than 256 segments in the
+//   batched kernel, whose teams may have 16 warps
 constexpr int32_t kMiscBytes = 320;
+constexpr int32_t kMiscBytesLong = 576;
 
 // Shared memory of one self contact while it is projected (batched kernel):
 // five 8-byte rows. A pool of nSt / 2 of them is the 20 nSt bytes that the
@@ -119,7 +122,7 @@ RP_HD inline RodLayout rodLayout(int32_t nP, int32_t nS, int32_t nSt, int32_t nB
     } else {
         L.slots = -1;
     }
-    L.misc = o;        o += kMiscBytes;
+    L.misc = o;        o += lean && nSt > 256 ? kMiscBytesLong : kMiscBytes;
     if (self && !lean) {
         L.centres = o; o += 16 * nSt;
         L.selfInt = o; o += 16 * nSt;

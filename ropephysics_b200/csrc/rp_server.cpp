@@ -187,7 +187,7 @@ struct rp_server {
     std::string workerError;
     rp_server_stats st{};
     double t0 = 0, busySince = -1;
-    int groupsN = 0, blocks = 0;
+    int groupsN = 0, blocks = 0, threads = 256;
     size_t smem = 0;
     bool dirty = true;
     std::thread worker;
@@ -312,33 +312,18 @@ bool rp_server::admit(Request& rq) {
 }
 
 bool rp_server::plan() {
-    std::vector<int32_t> ids, order, groups;
+    std::vector<int32_t> ids;
     for (auto& rq : running) ids.insert(ids.end(), rq->rodIds.begin(), rq->rodIds.end());
-    const bool comp = (cfg.precision & RP_PRECISION_COMPENSATED) != 0;
-    smem = rpx::planGroups(ids, hRods.data(), hTmpls.data(), 256, 1, comp, order, groups);
-    if (smem == rpx::kMisaligned) {
-        workerError = "internal: a rod's shared-memory layout is not 16-byte aligned";
+    rpx::BatchedShape shape;
+    if (rpx::planBatched(ids, hRods.data(), hTmpls.data(), 256, 1, cfg.precision, device, false, shape) != RP_OK) {
+        workerError = rp_last_error();
         return false;
     }
-    if (smem + rp::batchedStaticSmem() + 64 > rpx::optinSmem(device)) {
-        workerError = "a rod group exceeds shared memory";
-        return false;
-    }
-    if (rp::batchedReserveSmem(std::max<size_t>(smem, 1)) != cudaSuccess) {
-        cudaGetLastError();
-        workerError = "cannot reserve batched shared memory";
-        return false;
-    }
-    int perSm = 0;
-    if (rp::batchedOccupancy(256, smem, cfg.precision, &perSm) != cudaSuccess || perSm < 1) {
-        cudaGetLastError();
-        workerError = "batched kernel not resident";
-        return false;
-    }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const std::vector<int32_t>&order = shape.order, &groups = shape.groups;
     groupsN = int(groups.size() / 4);
-    blocks = std::max(1, std::min(groupsN, sms * perSm));
+    blocks = shape.blocks;
+    threads = shape.cta;
+    smem = shape.smem;
     cudaError_t e = cudaMemcpyAsync(dWork, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                                     stream);
     if (!e)
@@ -409,7 +394,7 @@ void rp_server::loop() {
         bp.numGroups = groupsN;
         bp.queue = dQueue;
         bp.blocks = blocks;
-        bp.threads = 256;
+        bp.threads = threads;
         bp.smemBytes = smem;
         lk.unlock();  // submitters may enqueue while the step runs
         cudaError_t e = rp::launchBatchedStep(A, bp, cfg.precision, stream);
