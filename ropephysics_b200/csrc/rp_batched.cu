@@ -54,21 +54,16 @@ __device__ __forceinline__ void teamSync(int team, int teamIdx) {
     }
 }
 
-// Order-preserving map of a float to an unsigned (negative values
-// reversed), so a warp's float min or max is one integer reduction
-// (redux.sync). Min and max are exact, so the result is one of the inputs.
-__device__ __forceinline__ unsigned orderedKey(float f) {
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float fromOrderedKey(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-}
+// Minimum and maximum over a warp (NaN operands are passed over, as fminf does)
 __device__ __forceinline__ float warpMax(float f) {
-    return fromOrderedKey(__reduce_max_sync(0xffffffffu, orderedKey(f)));
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f));
+    return r;
 }
 __device__ __forceinline__ float warpMin(float f) {
-    return fromOrderedKey(__reduce_min_sync(0xffffffffu, orderedKey(f)));
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f));
+    return r;
 }
 
 __device__ __forceinline__ float4 driveVelocityB(const DDrive& d, double t) {
@@ -174,8 +169,8 @@ struct TeamCtx {
 // pairs (j in J, k in K), two per lane: the per-pair sphere test of
 // querySelfSegment, then the shared narrow phase. The box test skips only
 // when box distance^2 > 1.0001 x bound^2 with every per-pair quantity bounded
-// by its block maximum (float max, add and multiply are monotone), so every
-// pair the sphere test keeps is reached.
+// from the rod's longest segment and the block's box (float max, add and
+// multiply are monotone), so every pair the sphere test keeps is reached.
 // A pair that passed the sphere test: the shared narrow phase, and for a
 // touching pair its bucket multiplicity, its count and its place in the pair
 // list (which holds nSt pairs; beyond that the count alone is kept and the
@@ -223,6 +218,10 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
     for (int J = warp; J < nBlk; J += warps) {
         const float4 jlo = S.blocks[2 * J], jhi = S.blocks[2 * J + 1];
         const int jmin = 8 * J;
+        // the sphere test's bound and slack for any pair of J with any block:
+        // cell = longest segment + 2 r, and the coordinates of J's centres
+        const float slackJ = 1e-6f * (1.0f + fmaxf(fabsf(jlo.x), fabsf(jhi.x)) + fmaxf(fabsf(jlo.y), fabsf(jhi.y)) +
+                                      fmaxf(fabsf(jlo.z), fabsf(jhi.z)));
         // this lane's segment of J for the pair tests against other blocks
         const int j = jmin + (wl & 7);
         const float4 cj = j < nSt ? S.centres[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -261,7 +260,7 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
                 const float gx = fmaxf(0.0f, fmaxf(klo.x - jhi.x, jlo.x - khi.x));
                 const float gy = fmaxf(0.0f, fmaxf(klo.y - jhi.y, jlo.y - khi.y));
                 const float gz = fmaxf(0.0f, fmaxf(klo.z - jhi.z, jlo.z - khi.z));
-                const float lim = (jlo.w + klo.w + twoR) * 1.001f + 1e-6f * jhi.w;
+                const float lim = cell * 1.001f + slackJ;
                 hit = !(gx * gx + gy * gy + gz * gz > lim * lim * 1.0001f);
             }
             unsigned m = __ballot_sync(0xffffffffu, hit);
@@ -804,64 +803,80 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 // One pass for both contact kinds: segment centres and half
                 // lengths, the longest segment (self-collision cell size), and the
                 // rod's bounding box (primitive culling).
+                //
+                // Bound: issue slots (17 % of a step of rods in free fall). Two
+                // segments a lane, so that a chain block of 8 takes two shuffle
+                // steps per bound instead of three and its inner particles are
+                // read once; the block's longest half and coordinate size are
+                // bounded in the count from the rod's longest segment and the
+                // box itself; a chain's box for the cull is its centres' box
+                // grown by half the longest segment; minima over the warp are one
+                // float redux each. 4096 x 64 over a floor, 80 substeps, 1.27 ->
+                // 1.19 ms; 4096 uneven rods with self-collision, 50 substeps, 6.93
+                // -> 6.55 ms.
                 float mx = 0.0f;
-                float lx = 3.0e38f, ly = 3.0e38f, lz = 3.0e38f;
-                float hx = -3.0e38f, hy = -3.0e38f, hz = -3.0e38f;
+                V3 lo{3.0e38f, 3.0e38f, 3.0e38f}, hi{-3.0e38f, -3.0e38f, -3.0e38f};
+                auto cover = [](V3& l, V3& h, V3 p) {
+                    l = V3{fminf(l.x, p.x), fminf(l.y, p.y), fminf(l.z, p.z)};
+                    h = V3{fmaxf(h.x, p.x), fmaxf(h.y, p.y), fmaxf(h.z, p.z)};
+                };
+                const bool boxOfCentres = self && T.chain;
                 if (self) {
                     // whole warps per round (team is a multiple of 32), so the
-                    // 8-lane shuffles bounding each chain block of 8 segments
+                    // 4-lane shuffles bounding each chain block of 8 segments
                     // always have every lane present; the counts are zeroed
                     // here too, so the count needs no barrier of its own
-                    for (int j0 = 0; j0 < nSt; j0 += team) {
-                        const int j = j0 + lane;
-                        float4 blo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f);
-                        float4 bhi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
-                        if (j < nSt) {
-                            const int p0 = T.chain ? j : V.g->sP0[j], p1 = T.chain ? j + 1 : V.g->sP1[j];
-                            const V3 a = v3(V.x[p0]), b = v3(V.x[p1]);
+                    for (int i0 = 0; 2 * i0 < nSt; i0 += team) {
+                        const int j = 2 * (i0 + lane);
+                        V3 bl{3.0e38f, 3.0e38f, 3.0e38f}, bh{-3.0e38f, -3.0e38f, -3.0e38f};
+                        auto centre = [&](int k, V3 a, V3 b) {
                             const float len = norm(b - a);
                             const V3 c = (a + b) * 0.5f;
-                            S.centres[j] = make_float4(c.x, c.y, c.z, 0.5f * len);
-                            S.segCount[j] = 0;
+                            S.centres[k] = make_float4(c.x, c.y, c.z, 0.5f * len);
+                            S.segCount[k] = 0;
                             mx = fmaxf(mx, len);
-                            blo = make_float4(c.x, c.y, c.z, 0.5f * len);
-                            bhi = make_float4(c.x, c.y, c.z, 1.0f + fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+                            cover(bl, bh, c);
+                        };
+                        if (j < nSt) {
+                            V3 a = v3(V.x[T.chain ? j : V.g->sP0[j]]), b = v3(V.x[T.chain ? j + 1 : V.g->sP1[j]]);
+                            centre(j, a, b);
+                            if (j + 1 < nSt) {
+                                a = T.chain ? b : v3(V.x[V.g->sP0[j + 1]]);
+                                b = v3(V.x[T.chain ? j + 2 : V.g->sP1[j + 1]]);
+                                centre(j + 1, a, b);
+                            }
                         }
+                        lo = V3{fminf(lo.x, bl.x), fminf(lo.y, bl.y), fminf(lo.z, bl.z)};
+                        hi = V3{fmaxf(hi.x, bh.x), fmaxf(hi.y, bh.y), fmaxf(hi.z, bh.z)};
 #pragma unroll
-                        for (int o = 1; o < 8; o <<= 1) {
-                            blo.x = fminf(blo.x, __shfl_xor_sync(0xffffffffu, blo.x, o));
-                            blo.y = fminf(blo.y, __shfl_xor_sync(0xffffffffu, blo.y, o));
-                            blo.z = fminf(blo.z, __shfl_xor_sync(0xffffffffu, blo.z, o));
-                            blo.w = fmaxf(blo.w, __shfl_xor_sync(0xffffffffu, blo.w, o));
-                            bhi.x = fmaxf(bhi.x, __shfl_xor_sync(0xffffffffu, bhi.x, o));
-                            bhi.y = fmaxf(bhi.y, __shfl_xor_sync(0xffffffffu, bhi.y, o));
-                            bhi.z = fmaxf(bhi.z, __shfl_xor_sync(0xffffffffu, bhi.z, o));
-                            bhi.w = fmaxf(bhi.w, __shfl_xor_sync(0xffffffffu, bhi.w, o));
+                        for (int o = 1; o < 4; o <<= 1) {
+                            bl.x = fminf(bl.x, __shfl_xor_sync(0xffffffffu, bl.x, o));
+                            bl.y = fminf(bl.y, __shfl_xor_sync(0xffffffffu, bl.y, o));
+                            bl.z = fminf(bl.z, __shfl_xor_sync(0xffffffffu, bl.z, o));
+                            bh.x = fmaxf(bh.x, __shfl_xor_sync(0xffffffffu, bh.x, o));
+                            bh.y = fmaxf(bh.y, __shfl_xor_sync(0xffffffffu, bh.y, o));
+                            bh.z = fmaxf(bh.z, __shfl_xor_sync(0xffffffffu, bh.z, o));
                         }
-                        if ((lane & 7) == 0 && j < nSt) {
-                            S.blocks[2 * (j >> 3)] = blo;
-                            S.blocks[2 * (j >> 3) + 1] = bhi;
+                        if ((lane & 3) == 0 && j < nSt) {
+                            S.blocks[2 * (j >> 3)] = f4(bl);
+                            S.blocks[2 * (j >> 3) + 1] = f4(bh);
                         }
                     }
+                    mx = warpMax(mx);
                 }
                 if (V.numPrims > 0) {
-                    for (int i = lane; i < nP; i += team) {
-                        const float4 p = V.x[i];
-                        lx = fminf(lx, p.x); ly = fminf(ly, p.y); lz = fminf(lz, p.z);
-                        hx = fmaxf(hx, p.x); hy = fmaxf(hy, p.y); hz = fmaxf(hz, p.z);
+                    if (!boxOfCentres) {
+                        lo = V3{3.0e38f, 3.0e38f, 3.0e38f};
+                        hi = V3{-3.0e38f, -3.0e38f, -3.0e38f};
+                        for (int i = lane; i < nP; i += team) cover(lo, hi, v3(V.x[i]));
                     }
+                    lo = V3{warpMin(lo.x), warpMin(lo.y), warpMin(lo.z)};
+                    hi = V3{warpMax(hi.x), warpMax(hi.y), warpMax(hi.z)};
                 }
-                mx = warpMax(mx);
-                lx = warpMin(lx);
-                ly = warpMin(ly);
-                lz = warpMin(lz);
-                hx = warpMax(hx);
-                hy = warpMax(hy);
-                hz = warpMax(hz);
-                if ((lane & 31) == 0) {
-                    float* row = red + 8 * (lane >> 5);
-                    row[0] = mx; row[1] = lx; row[2] = ly; row[3] = lz;
-                    row[4] = hx; row[5] = hy; row[6] = hz;
+                if (team > 32 && (lane & 31) == 0) {
+                    float4* const row = reinterpret_cast<float4*>(red + 8 * (lane >> 5));
+                    row[0] = make_float4(mx, lo.x, lo.y, lo.z);
+                    row[1] = f4(hi);
                 }
                 // reset before the barrier: the count below follows without one
                 if (lane == 0) {
@@ -872,14 +887,17 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 // every lane reduces the rows in the same order (max and min
                 // are exact), so every lane holds the same mask and cell size;
                 // lane 0 also publishes them for the later phases
-                for (int w = 0; w < (team >> 5); ++w) {
-                    const float* row = red + 8 * w;
-                    mx = fmaxf(mx, row[0]);
-                    lx = fminf(lx, row[1]); ly = fminf(ly, row[2]); lz = fminf(lz, row[3]);
-                    hx = fmaxf(hx, row[4]); hy = fmaxf(hy, row[5]); hz = fmaxf(hz, row[6]);
+                for (int w = 0; team > 32 && w < (team >> 5); ++w) {
+                    const float4* const row = reinterpret_cast<const float4*>(red + 8 * w);
+                    const float4 a = row[0], b = row[1];
+                    mx = fmaxf(mx, a.x);
+                    lo = V3{fminf(lo.x, a.y), fminf(lo.y, a.z), fminf(lo.z, a.w)};
+                    hi = V3{fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z)};
                 }
                 if (V.numPrims > 0) {
-                    maskNow = primitivesNearBox(V, V3{lx, ly, lz}, V3{hx, hy, hz});
+                    const float grow = boxOfCentres ? 0.5f * mx : 0.0f;
+                    const V3 g3{grow, grow, grow};
+                    maskNow = primitivesNearBox(V, lo - g3, hi + g3, lane & 31);
                     if (lane == 0) *primMask = maskNow;
                 }
                 cellNow = mx + 2.0f * V.radius;

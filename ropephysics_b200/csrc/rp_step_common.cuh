@@ -431,35 +431,42 @@ __device__ __forceinline__ void generateSlots(const RodView& V, int i, bool rege
 // distance from the box to a sphere that contains the primitive -- exceeds
 // the reach by a slack far above FP32 error, so no particle it drops could
 // have produced a contact: generation with the mask equals generation
-// without it.
-__device__ __forceinline__ unsigned long long primitivesNearBox(const RodView& V, V3 lo, V3 hi) {
+// without it. One warp, a primitive per lane; only the rows of a primitive
+// that its type needs are read.
+__device__ __forceinline__ unsigned long long primitivesNearBox(const RodView& V, V3 lo, V3 hi, int wl) {
     const V3 c = (lo + hi) * 0.5f;
     const V3 e = (hi - lo) * 0.5f;
     const float reach = V.radius + V.contactMargin;
     const float slack = 1e-3f * fabsf(reach) + 1e-4f +
                         1e-5f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + e.x + e.y + e.z);
     unsigned long long mask = 0ull;
-    for (int k = 0; k < V.numPrims && k < 64; ++k) {
-        const PrimF P = loadPrim(V.g->prims[k]);
-        bool near;
-        if (P.type == 0) {
-            const float s = dot(c - P.a, P.n) -
-                            (fabsf(P.n.x) * e.x + fabsf(P.n.y) * e.y + fabsf(P.n.z) * e.z);
-            near = s <= reach + slack;
-        } else {
-            V3 centre = P.a;
-            float rho = P.radius;
-            if (P.type == 2) {
-                centre = (P.a + P.b) * 0.5f;
-                rho = 0.5f * norm(P.b - P.a) + P.radius;
-            } else if (P.type == 3) {
-                rho = norm(P.h);
+    for (int k0 = 0; k0 < V.numPrims && k0 < 64; k0 += 32) {
+        const int k = k0 + wl;
+        bool near = false;
+        if (k < V.numPrims && k < 64) {
+            const float4* const row = reinterpret_cast<const float4*>(V.g->prims + k);
+            const float4 nt = row[2], ar = row[0];  // normal and type, point and radius
+            const int type = static_cast<int>(nt.w);
+            if (type == 0) {
+                const float s = dot(c - v3(ar), v3(nt)) -
+                                (fabsf(nt.x) * e.x + fabsf(nt.y) * e.y + fabsf(nt.z) * e.z);
+                near = s <= reach + slack;
+            } else {
+                V3 centre = v3(ar);
+                float rho = ar.w;
+                if (type == 2) {
+                    const V3 b = v3(row[1]);
+                    rho = 0.5f * norm(b - centre) + rho;
+                    centre = (centre + b) * 0.5f;
+                } else if (type == 3) {
+                    rho = norm(v3(row[3]));
+                }
+                const V3 d{fmaxf(fabsf(centre.x - c.x) - e.x, 0.0f), fmaxf(fabsf(centre.y - c.y) - e.y, 0.0f),
+                           fmaxf(fabsf(centre.z - c.z) - e.z, 0.0f)};
+                near = norm(d) - rho <= reach + slack;
             }
-            const V3 d{fmaxf(fabsf(centre.x - c.x) - e.x, 0.0f), fmaxf(fabsf(centre.y - c.y) - e.y, 0.0f),
-                       fmaxf(fabsf(centre.z - c.z) - e.z, 0.0f)};
-            near = norm(d) - rho <= reach + slack;
         }
-        if (near) mask |= 1ull << k;
+        mask |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, near)) << k0;
     }
     return mask;
 }
@@ -560,7 +567,7 @@ struct SelfScratch {
     float* cellSize;   // 1
     int32_t* live;     // 1
     int32_t* overflow; // 1
-    float4* blocks;    // chain blocks of 8 segments: {lo, max half}, {hi, max 1 + |c|_1}
+    float4* blocks;    // chain blocks of 8 segments: lowest and highest centre coordinates
 };
 
 // Narrow phase of one segment pair: closest points (u on a, w on b), their
