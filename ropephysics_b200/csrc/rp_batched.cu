@@ -110,9 +110,29 @@ __device__ int teamExclusiveScan(int32_t* a, int m, int lane, int team, int team
 // cell(j) whose hash is k's bucket hash(cell(k)): the cells, in the
 // reference's query order, at which its query meets k.
 __device__ __forceinline__ unsigned bucketCells(float4 cj, float4 ck, float cell, int table) {
-    const int cx = cellCoord(cj.x, cell), cy = cellCoord(cj.y, cell), cz = cellCoord(cj.z, cell);
-    const unsigned hk = hashCell(cellCoord(ck.x, cell), cellCoord(ck.y, cell), cellCoord(ck.z, cell), table);
+    bool ok = true;
+    const Divisor d = divisor(cell, recip(cell, ok));
+    ok = ok & (fmaxf(fmaxf(fabsf(cj.x), fabsf(cj.y)), fabsf(cj.z)) <= 0x1p60f) &
+         (fmaxf(fmaxf(fabsf(ck.x), fabsf(ck.y)), fabsf(ck.z)) <= 0x1p60f);
+    // cellCoord
+    auto coord = [&](float v) { return static_cast<int>(floorf(ok ? quotient(v, d) : v / cell)); };
+    const int cx = coord(cj.x), cy = coord(cj.y), cz = coord(cj.z);
+    const unsigned hk = hashCell(coord(ck.x), coord(ck.y), coord(ck.z), table);
+    const unsigned mask = unsigned(table) - 1u;
     unsigned m = 0u;
+    if ((unsigned(table) & mask) == 0u) {  // hashCell masks its hash
+        unsigned hx[3], hy[3], hz[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            hx[i] = unsigned(cx + i - 1) * 73856093u;
+            hy[i] = unsigned(cy + i - 1) * 19349663u;
+            hz[i] = (unsigned(cz + i - 1) * 83492791u) ^ hk;
+        }
+#pragma unroll
+        for (int t = 0; t < 27; ++t)
+            if (((hx[t % 3] ^ hy[t / 3 % 3] ^ hz[t / 9]) & mask) == 0u) m |= 1u << t;
+        return m;
+    }
     int t = 0;
     for (int dz = -1; dz <= 1; ++dz)
         for (int dy = -1; dy <= 1; ++dy)
@@ -123,8 +143,8 @@ __device__ __forceinline__ unsigned bucketCells(float4 cj, float4 ck, float cell
 
 // What a team needs about its rod beyond its shared-memory arrays: the fixed
 // global pointers, the colour tables, the drive, the self-contact scratch.
-// Lane 0 writes it once per rod into shared memory and every phase reads the
-// fields it uses, so the substep loop carries only the current phase's values
+// Lane 0 writes it once per rod into the rod's shared memory and every phase
+// reads the fields it uses, so the substep loop carries only the current phase's values
 // in registers (held in registers, these 64-bit pointers filled a third of
 // the register file and pushed the constraint arithmetic into spills). The
 // arrays in shared memory are not reached through it: pointers read back
@@ -163,14 +183,22 @@ struct TeamCtx {
 // every touching pair (j, k) is also appended to S.segStart as (j << 16) | k
 // (*C.numPairs(), zeroed by the caller, counts them; entries past nSt are not
 // stored).
-// Warp w of the team takes chain blocks J = w, w + warps, ...; its lanes test
-// 32 blocks K >= J at a time against J by box distance, and for each block
-// that can hold a pair within the sphere bound the warp runs the 64 segment
-// pairs (j in J, k in K), two per lane: the per-pair sphere test of
-// querySelfSegment, then the shared narrow phase. The box test skips only
-// when box distance^2 > 1.0001 x bound^2 with every per-pair quantity bounded
-// from the rod's longest segment and the block's box (float max, add and
-// multiply are monotone), so every pair the sphere test keeps is reached.
+// `reach` is the longest segment plus 2 r with the margins of the sphere test
+// of querySelfSegment (1.001 and 1e-6 of the coordinates' size, here of the
+// rod's largest), so a pair whose centres are farther apart fails that test;
+// `cell` is the longest segment plus 2 r. Pairs near along the chain are tested a segment per
+// lane, or ruled out by two distances; the others by chain blocks of 8
+// segments: box distance, then, for blocks within reach, the 64 pairs, two
+// per lane. Box and centre distances are monotone in float, so no pair the
+// sphere test keeps is missed. Pairs within reach wait in the warp's queue,
+// and the narrow phase runs on 32 of them at once.
+//
+// Bound: issue slots. In free fall three of five rounds a block went to near
+// pairs, which no rod passes that is not sharply bent. In settled rods two or
+// three lanes of a round pass, and the narrow phase run for those alone took
+// most of the count. 4096 uneven rods in free fall, 50 substeps, 6.55 -> 5.68 ms
+// (the count 10.6 -> 6.3 thousand cycles a rod and substep); 256 settled rods of
+// 16-512 2.02 -> 1.74 ms; 8 cables of 40-200, 20 substeps, 217 -> 157 us.
 // A pair that passed the sphere test: the shared narrow phase, and for a
 // touching pair its bucket multiplicity, its count and its place in the pair
 // list (which holds nSt pairs; beyond that the count alone is kept and the
@@ -195,11 +223,10 @@ __device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float
 }
 
 __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfScratch& S, int nSt, int gap,
-                                                  float radius, float cell, int lane, int team) {
+                                                  float cell, float reach, int lane, int team, int32_t* queue) {
     if (nSt <= gap) return;
     const int wl = lane & 31, warp = lane >> 5, warps = team >> 5;
     const int nBlk = (nSt + 7) >> 3;
-    const float twoR = 2.0f * radius;
     // This lane's pair of the block with itself, for the near pairs: the 28
     // pairs (a, b), a < b, of a block ordered by b - a descending, so the
     // pairs with b - a >= gap are a prefix (28 of them for gap 1, 15 for 3).
@@ -215,66 +242,99 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
             e -= 8 - d;
         }
     }
-    for (int J = warp; J < nBlk; J += warps) {
-        const float4 jlo = S.blocks[2 * J], jhi = S.blocks[2 * J + 1];
-        const int jmin = 8 * J;
-        // the sphere test's bound and slack for any pair of J with any block:
-        // cell = longest segment + 2 r, and the coordinates of J's centres
-        const float slackJ = 1e-6f * (1.0f + fmaxf(fabsf(jlo.x), fabsf(jhi.x)) + fmaxf(fabsf(jlo.y), fabsf(jhi.y)) +
-                                      fmaxf(fabsf(jlo.z), fabsf(jhi.z)));
-        // this lane's segment of J for the pair tests against other blocks
-        const int j = jmin + (wl & 7);
-        const float4 cj = j < nSt ? S.centres[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float scaleSlack = 1e-6f * (1.0f + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z));
-        // The per-pair test: the sphere test of querySelfSegment, then the
-        // narrow phase and the count for the pairs that pass.
-        auto testPair = [&](int pj, int pk, float4 pcj, float pslack) {
-            const float4 ck = S.centres[pk];
-            const float ddx = ck.x - pcj.x, ddy = ck.y - pcj.y, ddz = ck.z - pcj.z;
-            const float bound = pcj.w + ck.w + twoR;
-            const float plim = bound * 1.001f + pslack;
-            if (ddx * ddx + ddy * ddy + ddz * ddz > plim * plim) return;
-            countTouching(C, pj, pk, cell);
-        };
-        // Near pairs, with no box test (the boxes of J and J + 1 always
-        // meet): J against J + 1 in two rounds of 32, J against itself in one
-        // round over the pairs with b - a >= gap.
-        if (J + 1 < nBlk) {
-#pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-                const int k = 8 * (J + 1) + (wl >> 3) + 4 * h2;
-                if (j < nSt && k < nSt && k - j >= gap) testPair(j, k, cj, scaleSlack);
+    // The per-pair test of every lane that has a pair. The pairs that pass wait
+    // in the warp's queue for a full warp of them.
+    const unsigned below = (1u << wl) - 1u;
+    const float reach2 = reach * reach * 1.0001f;
+    int waiting = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        if (wl < waiting) countTouching(C, queue[wl] >> 16, queue[wl] & 0xffff, cell);
+        __syncwarp();
+        waiting = 0;
+    };
+    auto testPairs = [&](bool have, int j, int k) {
+        bool pass = false;
+        if (have) pass = !(norm2(v3(S.centres[k]) - v3(S.centres[j])) > reach2);
+        const unsigned m = __ballot_sync(0xffffffffu, pass);
+        if (m) {
+            if (waiting + __popc(m) > 32) flush();
+            if (pass) queue[waiting + __popc(m & below)] = (j << 16) | k;
+            waiting += __popc(m);
+        }
+    };
+    // Near pairs: between a block J and itself, J + 1 and J + 2, at most 23
+    // apart, 32 segments j at a time. Pairs exactly `gap` apart are tested as
+    // they are, a segment per lane. The others need no test where the centres 8
+    // and 18 segments on lie so far from j that those before and shortly
+    // behind them, each at most the longest segment from the next, are out of
+    // reach as well (the factor 1.002 is far above the rounding). A gap above 7
+    // is past what this covers: such rods test all near pairs.
+    const bool split = gap < 8;
+    const int near = split ? gap + 1 : gap;
+    const int last = nSt - 1;
+    const float step = (cell - 2.0f * C.V.radius) * 1.0001f;  // the longest segment
+    for (int j0 = 32 * warp; j0 < nSt; j0 += 32 * warps) {
+        unsigned clear = 0u;
+        if (split) {
+            const int j = j0 + wl;
+            testPairs(j + gap <= last, j, j + gap);
+            const V3 cj = v3(S.centres[min(j, last)]);
+            const int e8 = min(j + 8, last), e18 = min(j + 18, last);
+            const float d8 = norm2(v3(S.centres[e8]) - cj), d18 = norm2(v3(S.centres[e18]) - cj);
+            const float need8 = (reach + float(max(e8 - j - near, e8 < last ? 4 : 0)) * step) * 1.002f;
+            const float need18 = (reach + float(max(e18 - j - 13, e18 < last ? 5 : 0)) * step) * 1.002f;
+            clear = __ballot_sync(0xffffffffu, (e8 - j < near || d8 > need8 * need8) &&
+                                                   (e18 - j < 13 || d18 > need18 * need18));
+        }
+        if (clear == 0xffffffffu) continue;
+#pragma unroll 1
+        for (int J = j0 >> 3; J < min((j0 >> 3) + 4, nBlk); ++J, clear >>= 8) {
+            if ((clear & 0xffu) == 0xffu) continue;
+            // J against J + 1 and J + 2 in two rounds of 32 each, J against
+            // itself in one over the pairs with b - a >= near
+#pragma unroll 1
+            for (int round = 0; round < 5; ++round) {
+                const int j = 8 * J + (round < 4 ? wl & 7 : ta);
+                const int k = 8 * J + (round < 4 ? 8 + (wl >> 3) + 4 * round : tb);
+                testPairs((round < 4 || ta >= 0) && k < nSt && k - j >= near, j, k);
             }
         }
-        if (ta >= 0 && tb - ta >= gap && jmin + tb < nSt) {
-            const int j2 = jmin + ta;
-            const float4 cj2 = S.centres[j2];
-            testPair(j2, jmin + tb, cj2, 1e-6f * (1.0f + fabsf(cj2.x) + fabsf(cj2.y) + fabsf(cj2.z)));
-        }
-        // Blocks K >= J + 2, by box distance, 32 at a time.
-        for (int K0 = J + 2; K0 < nBlk; K0 += 32) {
+    }
+    // Far pairs: the boxes of two blocks J, J + 1 together against 32 blocks
+    // K >= J + 3 at a time, then each of the two against the blocks that are left.
+    for (int J0 = 2 * warp; J0 < nBlk; J0 += 2 * warps) {
+        const int J1 = min(J0 + 1, nBlk - 1);
+        const V3 l0 = v3(S.blocks[2 * J0]), h0 = v3(S.blocks[2 * J0 + 1]);
+        const V3 l1 = v3(S.blocks[2 * J1]), h1 = v3(S.blocks[2 * J1 + 1]);
+        const V3 lo{fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z)};
+        const V3 hi{fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z)};
+        auto apart = [](V3 al, V3 ah, V3 bl, V3 bh) {  // squared distance of two boxes
+            const float gx = fmaxf(0.0f, fmaxf(bl.x - ah.x, al.x - bh.x));
+            const float gy = fmaxf(0.0f, fmaxf(bl.y - ah.y, al.y - bh.y));
+            const float gz = fmaxf(0.0f, fmaxf(bl.z - ah.z, al.z - bh.z));
+            return gx * gx + gy * gy + gz * gz;
+        };
+        for (int K0 = J0 + 3; K0 < nBlk; K0 += 32) {
             const int K = K0 + wl;
             bool hit = false;
-            if (K < nBlk && min(8 * K + 7, nSt - 1) - jmin >= gap) {
-                const float4 klo = S.blocks[2 * K], khi = S.blocks[2 * K + 1];
-                const float gx = fmaxf(0.0f, fmaxf(klo.x - jhi.x, jlo.x - khi.x));
-                const float gy = fmaxf(0.0f, fmaxf(klo.y - jhi.y, jlo.y - khi.y));
-                const float gz = fmaxf(0.0f, fmaxf(klo.z - jhi.z, jlo.z - khi.z));
-                const float lim = cell * 1.001f + slackJ;
-                hit = !(gx * gx + gy * gy + gz * gz > lim * lim * 1.0001f);
-            }
-            unsigned m = __ballot_sync(0xffffffffu, hit);
-            while (m) {
+            if (K < nBlk) hit = !(apart(lo, hi, v3(S.blocks[2 * K]), v3(S.blocks[2 * K + 1])) > reach2);
+            for (unsigned m = __ballot_sync(0xffffffffu, hit); m; m &= m - 1u) {
                 const int Kh = K0 + __ffs(m) - 1;
-                m &= m - 1u;
-#pragma unroll
-                for (int h2 = 0; h2 < 2; ++h2) {
-                    const int k = 8 * Kh + (wl >> 3) + 4 * h2;
-                    if (j < nSt && k < nSt && k - j >= gap) testPair(j, k, cj, scaleSlack);
+                const V3 kl = v3(S.blocks[2 * Kh]), kh = v3(S.blocks[2 * Kh + 1]);
+#pragma unroll 1
+                for (int J = J0; J <= J0 + 1 && Kh >= J + 3; ++J) {
+                    if (apart(J == J0 ? l0 : l1, J == J0 ? h0 : h1, kl, kh) > reach2) continue;
+#pragma unroll 1
+                    for (int h2 = 0; h2 < 2; ++h2) {
+                        const int j = 8 * J + (wl & 7), k = 8 * Kh + (wl >> 3) + 4 * h2;
+                        testPairs(k < nSt && k - j >= near, j, k);
+                    }
                 }
             }
         }
     }
+    flush();
 }
 
 // Polls of the stage-in barrier before a lane gives up (each poll may wait a
@@ -283,8 +343,8 @@ constexpr int kStageTries = 1 << 20;
 // DArgs::errors bit of a rod whose state copy never completed
 constexpr int32_t kErrorStage = 2;
 
-// One context per team: a group holds at most eight rods.
-constexpr int kMaxTeamsPerCta = 8;
+static_assert(sizeof(TeamCtx) <= kContextBytes && alignof(TeamCtx) <= 16, "the layout's room for a team context");
+constexpr int kMaxWarps = 16;  // of a CTA
 
 // The order in which a filled pool is projected, by the team's first warp:
 // levels such that contacts of one level share no particle and every earlier
@@ -643,12 +703,14 @@ __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, in
 
 template <bool COMP, bool FP64>
 __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int team, int teamIdx,
-                       TeamCtx* ctxs) {
+                       int32_t* queue) {
     const DRod R = A.rods[r];
     const DTemplate T = A.tmpl[R.tmpl];
     const int nP = T.nP, nS = T.nS, nSt = T.nSt, nB = T.nB;
 
-    TeamCtx& C = ctxs[teamIdx];
+    const RodLayout L = rodLayout(nP, nS, nSt, nB, R.numPrims, R.selfCollision, R.hashTableSize,
+                                  R.selfCapacity, 1, COMP ? 1 : 0, A.slotsShared);
+    TeamCtx& C = *reinterpret_cast<TeamCtx*>(base + L.ctx);
     // The view of the rod's arrays lives in registers: its shared-memory
     // arrays are addressed from `base`, so the compiler reaches them with
     // shared-memory instructions through 32-bit addresses. The fixed global
@@ -661,8 +723,6 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     V.frictionScale = A.frictionScale[r];
     V.radius = R.radius;
     V.contactMargin = R.contactMargin;
-    const RodLayout L = rodLayout(nP, nS, nSt, nB, R.numPrims, R.selfCollision, R.hashTableSize,
-                                  R.selfCapacity, 1, COMP ? 1 : 0, A.slotsShared);
     V.q = reinterpret_cast<float4*>(base + L.q);
     V.qPrev = COMP ? A.gqPrev + R.sOff : reinterpret_cast<float4*>(base + L.qPrev);
     V.x = reinterpret_cast<float4*>(base + L.x);
@@ -798,7 +858,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
             }
             const bool regenerate = sub % interval == 0;
             unsigned long long maskNow = *primMask;  // this substep's primitive cull
-            float cellNow = 0.0f;                    // this substep's self-collision cell
+            float cellNow = 0.0f, sizeNow = 1.0f;    // this substep's self-collision cell, coordinate size
             if (regenerate && (V.numPrims > 0 || self)) {
                 // One pass for both contact kinds: segment centres and half
                 // lengths, the longest segment (self-collision cell size), and the
@@ -807,14 +867,13 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 // Bound: issue slots (17 % of a step of rods in free fall). Two
                 // segments a lane, so that a chain block of 8 takes two shuffle
                 // steps per bound instead of three and its inner particles are
-                // read once; the block's longest half and coordinate size are
-                // bounded in the count from the rod's longest segment and the
-                // box itself; a chain's box for the cull is its centres' box
+                // read once; the count bounds half lengths and coordinates by
+                // the rod's largest instead of the block's; a chain's box for the cull is its centres' box
                 // grown by half the longest segment; minima over the warp are one
                 // float redux each. 4096 x 64 over a floor, 80 substeps, 1.27 ->
                 // 1.19 ms; 4096 uneven rods with self-collision, 50 substeps, 6.93
                 // -> 6.55 ms.
-                float mx = 0.0f;
+                float mx = 0.0f, size = 1.0f;
                 V3 lo{3.0e38f, 3.0e38f, 3.0e38f}, hi{-3.0e38f, -3.0e38f, -3.0e38f};
                 auto cover = [](V3& l, V3& h, V3 p) {
                     l = V3{fminf(l.x, p.x), fminf(l.y, p.y), fminf(l.z, p.z)};
@@ -835,6 +894,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                             S.centres[k] = make_float4(c.x, c.y, c.z, 0.5f * len);
                             S.segCount[k] = 0;
                             mx = fmaxf(mx, len);
+                            size = fmaxf(size, 1.0f + fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
                             cover(bl, bh, c);
                         };
                         if (j < nSt) {
@@ -863,6 +923,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                         }
                     }
                     mx = warpMax(mx);
+                    size = warpMax(size);
                 }
                 if (V.numPrims > 0) {
                     if (!boxOfCentres) {
@@ -876,7 +937,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 if (team > 32 && (lane & 31) == 0) {
                     float4* const row = reinterpret_cast<float4*>(red + 8 * (lane >> 5));
                     row[0] = make_float4(mx, lo.x, lo.y, lo.z);
-                    row[1] = f4(hi);
+                    row[1] = make_float4(hi.x, hi.y, hi.z, size);
                 }
                 // reset before the barrier: the count below follows without one
                 if (lane == 0) {
@@ -891,6 +952,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     const float4* const row = reinterpret_cast<const float4*>(red + 8 * w);
                     const float4 a = row[0], b = row[1];
                     mx = fmaxf(mx, a.x);
+                    size = fmaxf(size, b.w);
                     lo = V3{fminf(lo.x, a.y), fminf(lo.y, a.z), fminf(lo.z, a.w)};
                     hi = V3{fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z)};
                 }
@@ -901,6 +963,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     if (lane == 0) *primMask = maskNow;
                 }
                 cellNow = mx + 2.0f * V.radius;
+                sizeNow = size;
                 if (self && lane == 0) {
                     if (sub == 0) *S.overflow = 0;
                     *S.cellSize = cellNow;  // for the fill pass, after later barriers
@@ -915,7 +978,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     // ---- count: contacts per segment, by chain blocks ----
                     // chain-block bounds and zeroed counts come from the centre pass
                     // the pair list takes segStart, which the hash path rebuilds
-                    countSelfByBlocks(C, S, nSt, C.selfGap, V.radius, cell, lane, team);
+                    countSelfByBlocks(C, S, nSt, C.selfGap, cell, cell * 1.001f + 1e-6f * sizeNow, lane, team, queue);
                     teamSync(team, teamIdx);
                     // team-uniform: shared words read after the barrier
                     const int pairs = *touching ? *numPairs : 0;
@@ -1091,7 +1154,7 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
                                                        int numGroups, int32_t* queue) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sGroup;
-    __shared__ TeamCtx ctxs[kMaxTeamsPerCta];
+    __shared__ int32_t queues[kMaxWarps][32];  // per warp: pairs that wait for the narrow phase
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) sGroup = atomicAdd(queue, 1);
@@ -1111,7 +1174,7 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
                                         Rk.hashTableSize, Rk.selfCapacity, 1, COMP ? 1 : 0, A.slotsShared)
                                   .bytes);
             }
-            runRod<COMP, FP64>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx, ctxs);
+            runRod<COMP, FP64>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx, queues[tid >> 5]);
         }
         __syncthreads();
     }

@@ -239,7 +239,7 @@ size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, cons
     int i = 0;
     while (i < n) {
         const int team = teamOf(order[i]);
-        const int perCta = std::min(8, cta / team);  // the kernel holds eight team contexts
+        const int perCta = std::min(8, cta / team);
         int cnt = 0;
         size_t smem = 0;
         while (i + cnt < n && cnt < perCta) {

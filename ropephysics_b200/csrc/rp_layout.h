@@ -28,6 +28,7 @@
 //   slots      [world contacts]                      32 x nP x numPrims (full, or lean
 //                                                    with slotsShared)
 //   misc       kMiscBytes (below)
+//   ctx        kContextBytes (lean): the team's context, TeamCtx
 //   self       full: centres 16 nSt, ints 16 nSt, hash 4 (table + 1) x 2,
 //              pool 64 x capacity, projection levels 3 x 4 (capacity + 1);
 //              lean: centres 16 nSt, chain-block bounds 32 x ceil(nSt / 8),
@@ -53,7 +54,7 @@ struct RodLayout {
     int32_t x, xPrev, v, force, kin, xComp, qComp;
     int32_t lamS, lamB;
     int32_t slots;
-    int32_t centres, selfInt, misc, hash, pool, levels, blocks;
+    int32_t centres, selfInt, misc, ctx, hash, pool, levels, blocks;
     int32_t bytes;
 };
 
@@ -67,6 +68,7 @@ struct RodLayout {
 //   batched kernel, whose teams may have 16 warps
 constexpr int32_t kMiscBytes = 320;
 constexpr int32_t kMiscBytesLong = 576;
+constexpr int32_t kContextBytes = 432;
 
 // Shared memory of one self contact while it is projected (batched kernel):
 // five 8-byte rows. A pool of nSt / 2 of them is the 20 nSt bytes that the
@@ -123,6 +125,11 @@ RP_HD inline RodLayout rodLayout(int32_t nP, int32_t nS, int32_t nSt, int32_t nB
         L.slots = -1;
     }
     L.misc = o;        o += lean && nSt > 256 ? kMiscBytesLong : kMiscBytes;
+    if (lean) {
+        L.ctx = o;     o += kContextBytes;
+    } else {
+        L.ctx = -1;
+    }
     if (self && !lean) {
         L.centres = o; o += 16 * nSt;
         L.selfInt = o; o += 16 * nSt;
@@ -154,7 +161,7 @@ RP_HD inline RodLayout rodLayout(int32_t nP, int32_t nS, int32_t nSt, int32_t nB
 // it); -1 marks a section the layout does not hold.
 RP_HD inline bool rodLayoutAligned(const RodLayout& L) {
     const int32_t s[] = {L.q, L.qPrev, L.omega, L.torque, L.x, L.xPrev, L.v, L.force, L.kin, L.xComp, L.qComp,
-                         L.lamS, L.lamB, L.slots, L.centres, L.selfInt, L.misc, L.hash, L.pool, L.levels,
+                         L.lamS, L.lamB, L.slots, L.centres, L.selfInt, L.misc, L.ctx, L.hash, L.pool, L.levels,
                          L.blocks, L.bytes};
     for (int32_t v : s)
         if (v != -1 && (v & 15) != 0) return false;
