@@ -483,6 +483,7 @@ rp_status launchStep(rp_batch* b, const rp_step_params* p, int steps) {
         plan.blocks = b->batchedBlocks;
         plan.threads = b->batchedThreads;
         plan.smemBytes = b->batchedSmem;
+        plan.anySelf = b->anySelf;
         e = rp::launchBatchedStep(A, plan, b->precision, b->stream);
         b->launches += 1;
     } else {
@@ -667,6 +668,7 @@ rp_status rp_batch_step_static_scratch(rp_batch* b, const rp_step_params* p) {
     plan.blocks = b->batchedBlocks;
     plan.threads = b->batchedThreads;
     plan.smemBytes = b->batchedSmem;
+    plan.anySelf = b->anySelf;
     // the two work-queue counters must be zero at launch; everything else is
     // written before it is read within the step
     RP_CUDA(cudaMemsetAsync(plan.queue, 0, 2 * sizeof(int32_t), b->stream));

@@ -154,6 +154,8 @@ struct TeamCtx {
     RodGlobals G;                   // the rod's fixed global pointers (V.g)
     RodView V;                      // copies of the view and scratch for the
     SelfScratch S;                  // separately compiled paths
+    float4* velocity;               // the rod's velocities in global memory
+    float4* omega;
     const int* sOrder;
     const int* bOrder;
     const int* sCol;
@@ -701,7 +703,7 @@ __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, in
     teamSync(team, teamIdx);
 }
 
-template <bool COMP, bool FP64>
+template <bool COMP, bool FP64, bool SELF>
 __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int team, int teamIdx,
                        int32_t* queue) {
     const DRod R = A.rods[r];
@@ -733,8 +735,6 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     // state arrays in global memory hold them between steps
     V.v = nullptr;
     V.omega = nullptr;
-    float4* const gv = A.v + R.pOff;
-    float4* const gw = A.omega + R.sOff;
     // multipliers: none at one iteration; else in global memory (L1/L2)
     V.lamS = A.iterations > 1 ? A.gLamS + R.stOff : nullptr;
     V.lamB = A.iterations > 1 ? A.gLamB + R.bOff : nullptr;
@@ -777,6 +777,8 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         G.force = A.force + R.pOff;
         G.kin = A.kinVel + R.pOff;
         G.torque = A.torque + R.sOff;
+        C.velocity = A.v + R.pOff;
+        C.omega = A.omega + R.sOff;
         C.V = V;  // for the rarely run, separately compiled paths
         G.view = &C.V;
         C.S = S;
@@ -842,7 +844,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     const V3 g{A.gx, A.gy, A.gz};
     const float h = A.h, invH2 = A.invH2;
     const int interval = A.contactInterval;
-    const bool self = R.selfCollision != 0;
+    const bool self = SELF && R.selfCollision != 0;
 
     const int stepsHere = A.stepsPerLaunch > 0 ? A.stepsPerLaunch : 1;
     for (int step = 0; step < stepsHere; ++step) {
@@ -1023,11 +1025,11 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
             // the prediction's own velocity is never read (the next update
             // replaces it), so velocities are in memory only between steps
             for (int i = lane; i < nP; i += team) {
-                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, h, A.linDecay) : gv[i];
+                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, h, A.linDecay) : C.velocity[i];
                 predictParticleFrom<COMP>(V, i, h, g, vi, nullptr);
             }
             for (int j = lane; j < nS; j += team) {
-                const float4 wj = sub > 0 ? finishedOmega<COMP>(V, j, h, A.angDecay) : gw[j];
+                const float4 wj = sub > 0 ? finishedOmega<COMP>(V, j, h, A.angDecay) : C.omega[j];
                 predictFrameFrom<COMP>(V, j, h, wj, nullptr);
             }
             teamSync(team, teamIdx);
@@ -1093,8 +1095,8 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 
         }
         // the step's last velocity update
-        for (int i = lane; i < nP; i += team) gv[i] = finishedVelocity<COMP>(V, i, h, A.linDecay);
-        for (int j = lane; j < nS; j += team) gw[j] = finishedOmega<COMP>(V, j, h, A.angDecay);
+        for (int i = lane; i < nP; i += team) C.velocity[i] = finishedVelocity<COMP>(V, i, h, A.linDecay);
+        for (int j = lane; j < nS; j += team) C.omega[j] = finishedOmega<COMP>(V, j, h, A.angDecay);
         teamSync(team, teamIdx);
 
         // ---- per-step bookkeeping ----
@@ -1117,26 +1119,27 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     }  // steps of this launch
 
     // ---- stage out: bulk copies from shared memory, then the outputs ----
+    const DRod& out = A.rods[r];  // read again: not worth registers through the steps
     // every lane's writes above reach the async proxy before lane 0 copies
     fenceProxyAsyncShared();
     teamSync(team, teamIdx);
     if (lane == 0) {
-        bulkStore(A.x + R.pOff, V.x, pBytes);
-        bulkStore(A.q + R.sOff, V.q, sBytes);
+        bulkStore(A.x + out.pOff, V.x, pBytes);
+        bulkStore(A.q + out.sOff, V.q, sBytes);
         if (COMP) {
-            bulkStore(A.xComp + R.pOff, V.xComp, pBytes);
-            bulkStore(A.qComp + R.sOff, V.qComp, sBytes);
+            bulkStore(A.xComp + out.pOff, V.xComp, pBytes);
+            bulkStore(A.qComp + out.sOff, V.qComp, sBytes);
         }
         bulkCommit();
     }
     if (V.numPrims > 0 && A.contactState) {
         const int slots = nP * V.numPrims;
         for (int s = lane; s < slots; s += team)
-            A.contactState[R.slotOff + s] = ((*primMask >> (s % V.numPrims)) & 1ull) ? static_cast<uint8_t>(V.slots[s].state) : uint8_t(0);
+            A.contactState[out.slotOff + s] = ((*primMask >> (s % V.numPrims)) & 1ull) ? static_cast<uint8_t>(V.slots[s].state) : uint8_t(0);
     }
     if (self) {
         const int live = *S.live;
-        for (int c = lane; c < live; c += team) A.selfPairs[R.poolOff + c] = S.pool[c].seg;
+        for (int c = lane; c < live; c += team) A.selfPairs[out.poolOff + c] = S.pool[c].seg;
     }
     if (lane == 0) {
         if (self) A.selfCount[r] = *S.live;
@@ -1149,7 +1152,11 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     fenceProxyAsyncShared();
 }
 
-template <bool COMP, bool FP64>
+// SELF: some rod of the launch collides with itself. Launches without run an
+// instance without that code, which spills 32 bytes where this one spills 336
+// (loads, reference order) at the 128 registers that two 256-thread CTAs leave:
+// 4096 rods of 64 over a floor, 80 substeps, 1.25 -> 1.13 ms.
+template <bool COMP, bool FP64, bool SELF>
 __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* __restrict__ groups,
                                                        int numGroups, int32_t* queue) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1174,7 +1181,7 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
                                         Rk.hashTableSize, Rk.selfCapacity, 1, COMP ? 1 : 0, A.slotsShared)
                                   .bytes);
             }
-            runRod<COMP, FP64>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx, queues[tid >> 5]);
+            runRod<COMP, FP64, SELF>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx, queues[tid >> 5]);
         }
         __syncthreads();
     }
@@ -1191,33 +1198,27 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
     }
 }
 
-template <bool COMP, bool FP64>
-cudaError_t launchB(const DArgs& a, const BatchedPlan& p, cudaStream_t s) {
-    kBatchedStep<COMP, FP64><<<p.blocks, p.threads, p.smemBytes, s>>>(a, p.groups, p.numGroups, p.queue);
-    return cudaGetLastError();
+using Kernel = void (*)(DArgs, const int32_t*, int, int32_t*);
+
+// The instance for a precision and for launches with or without
+// self-collision.
+Kernel instance(int precision, bool self) {
+    const bool comp = (precision & 1) != 0, fp64 = (precision & 2) != 0;
+    if (self) {
+        if (comp) return fp64 ? kBatchedStep<true, true, true> : kBatchedStep<true, false, true>;
+        return fp64 ? kBatchedStep<false, true, true> : kBatchedStep<false, false, true>;
+    }
+    if (comp) return fp64 ? kBatchedStep<true, true, false> : kBatchedStep<true, false, false>;
+    return fp64 ? kBatchedStep<false, true, false> : kBatchedStep<false, false, false>;
 }
 
 }  // namespace
 
 cudaError_t launchBatchedStep(const DArgs& a, const BatchedPlan& p, int precision, cudaStream_t s) {
     if (p.numGroups <= 0) return cudaSuccess;
-    const bool comp = (precision & 1) != 0, fp64 = (precision & 2) != 0;
-    if (comp) return fp64 ? launchB<true, true>(a, p, s) : launchB<true, false>(a, p, s);
-    return fp64 ? launchB<false, true>(a, p, s) : launchB<false, false>(a, p, s);
+    instance(precision, p.anySelf)<<<p.blocks, p.threads, p.smemBytes, s>>>(a, p.groups, p.numGroups, p.queue);
+    return cudaGetLastError();
 }
-
-namespace {
-cudaError_t setMaxDynamicSmem_batched(int b) {
-    cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kBatchedStep<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b)))
-        return e;
-    if ((e = cudaFuncSetAttribute(kBatchedStep<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b)))
-        return e;
-    if ((e = cudaFuncSetAttribute(kBatchedStep<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b)))
-        return e;
-    return cudaFuncSetAttribute(kBatchedStep<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-}
-}  // namespace
 
 // The attribute belongs to the kernel, not to a batch: it only ever grows
 // (per device), so a later, smaller plan never shrinks what an earlier batch
@@ -1232,32 +1233,29 @@ cudaError_t batchedReserveSmem(size_t bytes) {
     std::lock_guard<std::mutex> g(mu);
     const int want = static_cast<int>(bytes);
     if (want <= reserved[dev]) return cudaSuccess;
-    e = setMaxDynamicSmem_batched(want);
-    if (e == cudaSuccess) reserved[dev] = want;
-    return e;
+    for (int i = 0; i < 8; ++i)
+        if ((e = cudaFuncSetAttribute(instance(i & 3, (i & 4) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      want)) != cudaSuccess)
+            return e;
+    reserved[dev] = want;
+    return cudaSuccess;
 }
 
-// The kernel's static shared memory (team contexts, the group word): the
+// The kernel's static shared memory (the warps' queues, the group word): the
 // dynamic part of a plan may use the opt-in limit minus this.
 size_t batchedStaticSmem() {
     size_t most = 0;
     cudaFuncAttributes a;
-    if (cudaFuncGetAttributes(&a, kBatchedStep<false, false>) == cudaSuccess) most = std::max(most, a.sharedSizeBytes);
-    if (cudaFuncGetAttributes(&a, kBatchedStep<false, true>) == cudaSuccess) most = std::max(most, a.sharedSizeBytes);
-    if (cudaFuncGetAttributes(&a, kBatchedStep<true, false>) == cudaSuccess) most = std::max(most, a.sharedSizeBytes);
-    if (cudaFuncGetAttributes(&a, kBatchedStep<true, true>) == cudaSuccess) most = std::max(most, a.sharedSizeBytes);
+    for (int i = 0; i < 8; ++i)
+        if (cudaFuncGetAttributes(&a, instance(i & 3, (i & 4) != 0)) == cudaSuccess)
+            most = std::max(most, a.sharedSizeBytes);
     cudaGetLastError();
     return most;
 }
 
-cudaError_t batchedOccupancy(int threads, size_t smem, int precision, int* perSm) {
+cudaError_t batchedOccupancy(int threads, size_t smem, int precision, bool anySelf, int* perSm) {
     // the instance the launch will use: register counts differ between them
-    const bool comp = (precision & 1) != 0, fp64 = (precision & 2) != 0;
-    if (comp)
-        return fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, kBatchedStep<true, true>, threads, smem)
-                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, kBatchedStep<true, false>, threads, smem);
-    return fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, kBatchedStep<false, true>, threads, smem)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, kBatchedStep<false, false>, threads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, instance(precision, anySelf), threads, smem);
 }
 
 }  // namespace rp

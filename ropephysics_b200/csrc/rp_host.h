@@ -58,6 +58,7 @@ struct BatchedShape {
     int blocks = 1;                      // persistent grid
     size_t smem = 0;                     // dynamic shared memory per CTA
     int slotsShared = 0;                 // world contact slots in shared memory
+    bool anySelf = false;                // a rod collides with itself
 };
 rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
                       int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out);

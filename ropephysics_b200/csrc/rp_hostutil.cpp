@@ -285,8 +285,8 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
         int per1 = 0, per2 = 0;
         if (smem2 != kMisaligned && smem2 + fixed <= optin &&
             rp::batchedReserveSmem(std::max(smem2, out.smem)) == cudaSuccess &&
-            rp::batchedOccupancy(cta, out.smem, precision, &per1) == cudaSuccess &&
-            rp::batchedOccupancy(cta, smem2, precision, &per2) == cudaSuccess && per2 >= per1 && per2 >= 1) {
+            rp::batchedOccupancy(cta, out.smem, precision, out.anySelf, &per1) == cudaSuccess &&
+            rp::batchedOccupancy(cta, smem2, precision, out.anySelf, &per2) == cudaSuccess && per2 >= per1 && per2 >= 1) {
             out.smem = smem2;
             out.order.swap(order2);
             out.groups.swap(groups2);
@@ -302,7 +302,7 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
         cudaGetLastError();
         return fail(RP_ERR_SHARED_MEMORY, "cannot opt into the batched shared memory");
     }
-    if (rp::batchedOccupancy(cta, out.smem, precision, perSm) != cudaSuccess || *perSm < 1) {
+    if (rp::batchedOccupancy(cta, out.smem, precision, out.anySelf, perSm) != cudaSuccess || *perSm < 1) {
         cudaGetLastError();
         return fail(RP_ERR_SHARED_MEMORY, "batched kernel cannot be resident with this group size");
     }
@@ -333,6 +333,8 @@ rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, 
                       int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out) {
     const size_t optin = optinSmem(device);
     int sms = 0, perSm = 0;
+    out.anySelf = false;
+    for (int32_t r : rodIds) out.anySelf = out.anySelf || rods[r].selfCollision != 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (cta == 256 && pairsPerThread == 1) {
         int longest = 0;

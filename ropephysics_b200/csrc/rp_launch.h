@@ -22,6 +22,7 @@ struct BatchedPlan {
     int32_t blocks;         // persistent grid size
     int32_t threads;        // CTA size
     size_t smemBytes;       // dynamic shared memory per CTA
+    bool anySelf;           // a rod of the launch collides with itself
 };
 cudaError_t launchBatchedStep(const DArgs& a, const BatchedPlan& plan, int precision,
                               cudaStream_t stream);
@@ -29,7 +30,7 @@ cudaError_t batchedReserveSmem(size_t bytes);
 // Static shared memory of the batched kernel (bytes), which a plan's dynamic
 // shared memory must leave room for under the opt-in limit.
 size_t batchedStaticSmem();
-cudaError_t batchedOccupancy(int threads, size_t smemBytes, int precision, int* blocksPerSm);
+cudaError_t batchedOccupancy(int threads, size_t smemBytes, int precision, bool anySelf, int* blocksPerSm);
 
 // Address and size of this device's static scratch array (looked up on the
 // first call per device, with that device current).

@@ -189,6 +189,7 @@ struct rp_server {
     double t0 = 0, busySince = -1;
     int groupsN = 0, blocks = 0, threads = 256;
     size_t smem = 0;
+    bool anySelf = false;
     bool dirty = true;
     std::thread worker;
 
@@ -324,6 +325,7 @@ bool rp_server::plan() {
     blocks = shape.blocks;
     threads = shape.cta;
     smem = shape.smem;
+    anySelf = shape.anySelf;
     cudaError_t e = cudaMemcpyAsync(dWork, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                                     stream);
     if (!e)
@@ -396,6 +398,7 @@ void rp_server::loop() {
         bp.blocks = blocks;
         bp.threads = threads;
         bp.smemBytes = smem;
+        bp.anySelf = anySelf;
         lk.unlock();  // submitters may enqueue while the step runs
         cudaError_t e = rp::launchBatchedStep(A, bp, cfg.precision, stream);
         if (!e) e = cudaStreamSynchronize(stream);
