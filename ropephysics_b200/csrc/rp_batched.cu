@@ -141,6 +141,8 @@ __device__ __forceinline__ unsigned bucketCells(float4 cj, float4 ck, float cell
     return m;
 }
 
+constexpr int kMaxWarps = 16;  // of a CTA
+
 // What a team needs about its rod beyond its shared-memory arrays: the fixed
 // global pointers, the colour tables, the drive, the self-contact scratch.
 // Lane 0 writes it once per rod into the rod's shared memory and every phase
@@ -160,6 +162,8 @@ struct TeamCtx {
     const int* bOrder;
     const int* sCol;
     const int* bCol;
+    int32_t rod;                    // its index
+    int32_t sColors, bColors;
     int32_t nP, nSt;
     int32_t table, selfGap, selfCapacity;
     float selfFriction;
@@ -210,7 +214,7 @@ __device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                        v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
+                                        v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
     if (P.separation >= 0.0f) return;
     const unsigned cells = bucketCells(S.centres[j], S.centres[k], cell, C.table);
     if (cells) {
@@ -225,7 +229,8 @@ __device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float
 }
 
 __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfScratch& S, int nSt, int gap,
-                                                  float cell, float reach, int lane, int team, int32_t* queue) {
+                                                  float cell, float reach, int lane, int team) {
+    __shared__ int32_t queues[kMaxWarps][32];  // per warp: pairs that wait for the narrow phase
     if (nSt <= gap) return;
     const int wl = lane & 31, warp = lane >> 5, warps = team >> 5;
     const int nBlk = (nSt + 7) >> 3;
@@ -247,6 +252,7 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
     // The per-pair test of every lane that has a pair. The pairs that pass wait
     // in the warp's queue for a full warp of them.
     const unsigned below = (1u << wl) - 1u;
+    int32_t* const queue = queues[threadIdx.x >> 5];
     const float reach2 = reach * reach * 1.0001f;
     int waiting = 0;
     auto flush = [&]() {
@@ -275,7 +281,7 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
     const bool split = gap < 8;
     const int near = split ? gap + 1 : gap;
     const int last = nSt - 1;
-    const float step = (cell - 2.0f * C.V.radius) * 1.0001f;  // the longest segment
+    const float step = (cell - 2.0f * C.V.g->radius) * 1.0001f;  // the longest segment
     for (int j0 = 32 * warp; j0 < nSt; j0 += 32 * warps) {
         unsigned clear = 0u;
         if (split) {
@@ -346,7 +352,6 @@ constexpr int kStageTries = 1 << 20;
 constexpr int32_t kErrorStage = 2;
 
 static_assert(sizeof(TeamCtx) <= kContextBytes && alignof(TeamCtx) <= 16, "the layout's room for a team context");
-constexpr int kMaxWarps = 16;  // of a CTA
 
 // The order in which a filled pool is projected, by the team's first warp:
 // levels such that contacts of one level share no particle and every earlier
@@ -365,7 +370,7 @@ constexpr int kMaxWarps = 16;  // of a CTA
 //
 // An entry that indexes outside the rod or was left unwritten cuts the pool
 // before it and is reported; it is never dereferenced.
-__device__ __noinline__ void orderPool(const TeamCtx& C, int live, int precision, int32_t* errorWord, int lane) {
+__device__ __forceinline__ void orderPool(const TeamCtx& C, int live, int precision, int32_t* errorWord, int lane) {
     constexpr unsigned kAll = 0xffffffffu;
     const SelfScratch& S = C.S;
     const int nP = C.nP;
@@ -473,9 +478,7 @@ __device__ __noinline__ void orderPool(const TeamCtx& C, int live, int precision
 // The pool fill of a substep on which some segment pair touches: the
 // reference's hash (a stable counting sort) and its fill pass in bucket order.
 // For pools that the pair list cannot give (more than nSt touching pairs).
-// Not inlined: inlined its registers would count against every phase of the
-// substep loop.
-__device__ __noinline__ void fillSelfPool(const TeamCtx& C, float cell, int live, int lane, int team,
+__device__ __forceinline__ void fillSelfPool(const TeamCtx& C, float cell, int live, int lane, int team,
                                           int teamIdx) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
@@ -536,7 +539,7 @@ __device__ __noinline__ void fillSelfPool(const TeamCtx& C, float cell, int live
 // returns the reference's count of entries. The pair list is
 // S.segStart[0..numPairs), numPairs <= 32, with the cells in S.sorted; S.segCount
 // holds the pairs' cells afterwards.
-__device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int lane) {
+__device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int lane) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const bool mine = lane < numPairs;
@@ -554,7 +557,7 @@ __device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int la
     __syncwarp();
     if (mine) {
         const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
+                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
         // entries of the pairs of earlier segments
         int before = 0;
         for (int q = 0; q < numPairs; ++q)
@@ -587,7 +590,7 @@ __device__ __noinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int la
 // 1500-2200 segments at 20 substeps 32.4 -> 10.5 ms, 256 of 16-512 at 50
 // substeps 8.53 -> 2.08 ms, and rods in free fall, which touch now and then,
 // 4096 of 16-512, 7.65 -> 6.93 ms.
-__device__ __noinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, int lane, int team, int teamIdx) {
+__device__ __forceinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, int lane, int team, int teamIdx) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const int nSt = C.nSt;
@@ -607,7 +610,7 @@ __device__ __noinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, in
         if (before >= C.selfCapacity) continue;
         const unsigned cells = unsigned(cellsOf[p]);
         const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.radius);
+                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
         for (unsigned rest = cells; rest; rest &= rest - 1u) {
             const int t = __ffs(rest) - 1;
             const unsigned below = (1u << t) - 1u;
@@ -620,6 +623,32 @@ __device__ __noinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, in
         }
     }
     return total;
+}
+
+// The pool of a substep on which some pair touches, and its order. One call:
+// each function called from the substep loop makes the loop's registers live
+// across it.
+__device__ __noinline__ void buildPool(const TeamCtx& C, float cell, int precision, int32_t* errorWord, int lane,
+                                       int team, int teamIdx) {
+    const SelfScratch& S = C.S;
+    const int pairs = *C.numPairs(), nSt = C.nSt;
+    int total = 0;
+    if (pairs <= 32 && pairs <= nSt) {
+        if (lane < 32) total = poolFromPairs(C, pairs, lane);
+    } else if (pairs <= nSt) {
+        total = poolFromManyPairs(C, pairs, lane, team, teamIdx);
+    } else {
+        for (int j = lane; j < nSt; j += team) S.segStart[j] = S.segCount[j];
+        teamSync(team, teamIdx);
+        total = teamExclusiveScan(S.segStart, nSt, lane, team, teamIdx, C.partial());
+        fillSelfPool(C, cell, min(total, C.selfCapacity), lane, team, teamIdx);
+    }
+    if (lane == 0) {
+        *S.live = min(total, C.selfCapacity);
+        if (total > C.selfCapacity) *S.overflow += total - C.selfCapacity;
+    }
+    teamSync(team, teamIdx);  // pool written, positions read: the prediction may start
+    if (lane < 32) orderPool(C, *S.live, precision, errorWord, lane);
 }
 
 // Contact c of the pool into its place of the compact, level-major rows in
@@ -657,7 +686,7 @@ __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, in
     float4* const xComp = COMP ? reinterpret_cast<float4*>(shared(V.xComp)) : nullptr;
     float2* const rows = reinterpret_cast<float2*>(shared(S.centres));
     const int32_t* const ends = reinterpret_cast<const int32_t*>(shared(S.segCount)) + live;
-    const float friction = C.selfFriction * V.frictionScale;
+    const float friction = C.selfFriction * V.g->frictionScale;
     const bool oneWarp = live <= 32 * levels;
     const int stride = oneWarp ? 32 : team;
     if (lane < stride) {
@@ -704,8 +733,7 @@ __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, in
 }
 
 template <bool COMP, bool FP64, bool SELF>
-__device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int team, int teamIdx,
-                       int32_t* queue) {
+__device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int team, int teamIdx) {
     const DRod R = A.rods[r];
     const DTemplate T = A.tmpl[R.tmpl];
     const int nP = T.nP, nS = T.nS, nSt = T.nSt, nB = T.nB;
@@ -721,10 +749,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     RodView V;
     V.g = &C.G;
     V.numPrims = R.numPrims;
-    V.complianceScale = A.complianceScale[r];
-    V.frictionScale = A.frictionScale[r];
-    V.radius = R.radius;
-    V.contactMargin = R.contactMargin;
+    V.softness = A.invH2 * A.complianceScale[r];
     V.q = reinterpret_cast<float4*>(base + L.q);
     V.qPrev = COMP ? A.gqPrev + R.sOff : reinterpret_cast<float4*>(base + L.qPrev);
     V.x = reinterpret_cast<float4*>(base + L.x);
@@ -752,8 +777,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     S.cellSize = reinterpret_cast<float*>(misc);
     S.live = misc + 1;
     S.overflow = misc + 2;
-    S.blocks = reinterpret_cast<float4*>(base + L.blocks);
-    int32_t* partial = misc + 16;  // one per warp of the team
+    S.blocks = S.centres + nSt;
     int32_t* numLevels = misc + 3;
     unsigned long long* primMask = reinterpret_cast<unsigned long long*>(misc + 12);
     int32_t* touching = misc + 14;
@@ -777,6 +801,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         G.force = A.force + R.pOff;
         G.kin = A.kinVel + R.pOff;
         G.torque = A.torque + R.sOff;
+        G.radius = R.radius;
+        G.contactMargin = R.contactMargin;
+        G.frictionScale = A.frictionScale[r];
         C.velocity = A.v + R.pOff;
         C.omega = A.omega + R.sOff;
         C.V = V;  // for the rarely run, separately compiled paths
@@ -792,6 +819,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         C.bOrder = A.tOrder + T.bOrderOff;
         C.sCol = A.tColorStart + T.sColorOff;
         C.bCol = A.tColorStart + T.bColorOff;
+        C.sColors = T.sColors;
+        C.bColors = T.bColors;
+        C.rod = r;
         *numLevels = 0;
         *primMask = ~0ull;
         // simulated time of this rod, advanced per step exactly as the
@@ -842,15 +872,17 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     }
 
     const V3 g{A.gx, A.gy, A.gz};
-    const float h = A.h, invH2 = A.invH2;
+    const float h = A.h;
     const int interval = A.contactInterval;
     const bool self = SELF && R.selfCollision != 0;
+    // bits 0 and 1: even/odd stretch and bend colours of a chain; bit 2: a chain
+    const int order = T.chain ? (T.evenOdd & 3) | 4 : 0;
 
     const int stepsHere = A.stepsPerLaunch > 0 ? A.stepsPerLaunch : 1;
     for (int step = 0; step < stepsHere; ++step) {
         if (lane == 0) {
-            if (C.driveP >= 0) V.g->kin[C.driveP] = driveVelocityB(A.drives[r], C.tRod);
-            if (C.wayP >= 0) V.g->kin[C.wayP] = waypointVelocity(A.waypoints[r], C.wayStep + step);
+            if (C.driveP >= 0) V.g->kin[C.driveP] = driveVelocityB(A.drives[C.rod], C.tRod);
+            if (C.wayP >= 0) V.g->kin[C.wayP] = waypointVelocity(A.waypoints[C.rod], C.wayStep + step);
         }
         teamSync(team, teamIdx);
         for (int sub = 0; sub < A.substeps; ++sub) {
@@ -881,7 +913,8 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     l = V3{fminf(l.x, p.x), fminf(l.y, p.y), fminf(l.z, p.z)};
                     h = V3{fmaxf(h.x, p.x), fmaxf(h.y, p.y), fmaxf(h.z, p.z)};
                 };
-                const bool boxOfCentres = self && T.chain;
+                const bool chain = (order & 4) != 0;
+                const bool boxOfCentres = self && chain;
                 if (self) {
                     // whole warps per round (team is a multiple of 32), so the
                     // 4-lane shuffles bounding each chain block of 8 segments
@@ -900,11 +933,11 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                             cover(bl, bh, c);
                         };
                         if (j < nSt) {
-                            V3 a = v3(V.x[T.chain ? j : V.g->sP0[j]]), b = v3(V.x[T.chain ? j + 1 : V.g->sP1[j]]);
+                            V3 a = v3(V.x[chain ? j : V.g->sP0[j]]), b = v3(V.x[chain ? j + 1 : V.g->sP1[j]]);
                             centre(j, a, b);
                             if (j + 1 < nSt) {
-                                a = T.chain ? b : v3(V.x[V.g->sP0[j + 1]]);
-                                b = v3(V.x[T.chain ? j + 2 : V.g->sP1[j + 1]]);
+                                a = chain ? b : v3(V.x[V.g->sP0[j + 1]]);
+                                b = v3(V.x[chain ? j + 2 : V.g->sP1[j + 1]]);
                                 centre(j + 1, a, b);
                             }
                         }
@@ -964,7 +997,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     maskNow = primitivesNearBox(V, lo - g3, hi + g3, lane & 31);
                     if (lane == 0) *primMask = maskNow;
                 }
-                cellNow = mx + 2.0f * V.radius;
+                cellNow = mx + 2.0f * V.g->radius;
                 sizeNow = size;
                 if (self && lane == 0) {
                     if (sub == 0) *S.overflow = 0;
@@ -980,33 +1013,14 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                     // ---- count: contacts per segment, by chain blocks ----
                     // chain-block bounds and zeroed counts come from the centre pass
                     // the pair list takes segStart, which the hash path rebuilds
-                    countSelfByBlocks(C, S, nSt, C.selfGap, cell, cell * 1.001f + 1e-6f * sizeNow, lane, team, queue);
+                    countSelfByBlocks(C, S, nSt, C.selfGap, cell, cell * 1.001f + 1e-6f * sizeNow, lane, team);
                     teamSync(team, teamIdx);
                     // team-uniform: shared words read after the barrier
-                    const int pairs = *touching ? *numPairs : 0;
-                    int total = 0;
-                    if (pairs > 0 && pairs <= nSt) {
-                        if (pairs <= 32) {
-                            if (lane < 32)
-                                total = poolFromPairs(C, pairs, lane);
-                        } else {
-                            total = poolFromManyPairs(C, pairs, lane, team, teamIdx);
-                        }
-                    } else if (pairs > 0) {
-                        for (int j = lane; j < nSt; j += team) S.segStart[j] = S.segCount[j];
-                        teamSync(team, teamIdx);
-                        total = teamExclusiveScan(S.segStart, nSt, lane, team, teamIdx, partial);
-                        fillSelfPool(C, cell, min(total, C.selfCapacity), lane, team, teamIdx);
-                    }
-                    if (lane == 0) {
-                        *S.live = min(total, C.selfCapacity);
-                        if (total > C.selfCapacity) *S.overflow += total - C.selfCapacity;
-                        if (pairs == 0) *numLevels = 0;
-                    }
-                    if (pairs > 0) {  // team-uniform
-                        teamSync(team, teamIdx);  // pool written, positions read: the prediction may start
-                        if (lane < 32)
-                            orderPool(C, *S.live, A.precision, A.errors ? A.errors + r : nullptr, lane);
+                    if (*touching) {
+                        buildPool(C, cell, A.precision, A.errors ? A.errors + C.rod : nullptr, lane, team, teamIdx);
+                    } else if (lane == 0) {
+                        *S.live = 0;
+                        *numLevels = 0;
                     }
                 } else {
                     float2* const lam = reinterpret_cast<float2*>(S.centres) + 4 * *S.live;
@@ -1042,26 +1056,26 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 // a chain coloured even/odd: constraint k of colour c is
                 // k = 2 i + c with particles k, k+1 and frames k, k+1, so no
                 // index is loaded; same constraints, same arithmetic
-                if (T.chain && (T.evenOdd & 1)) {
+                if (order & 1) {
                     for (int c = 0; c < 2; ++c) {
                         for (int k = 2 * lane + c; k < nSt; k += 2 * team)
-                            projectStretchAt<COMP>(V, k, k, k + 1, k, invH2);
+                            projectStretchAt<COMP>(V, k, k, k + 1, k);
                         teamSync(team, teamIdx);
                     }
                 } else {
-                    for (int c = 0; c < T.sColors; ++c) {
+                    for (int c = 0; c < C.sColors; ++c) {
                         for (int ci = sCol[c] + lane; ci < sCol[c + 1]; ci += team)
-                            projectStretchOne<COMP>(V, sOrder[ci], invH2);
+                            projectStretchOne<COMP>(V, sOrder[ci]);
                         teamSync(team, teamIdx);
                     }
                 }
-                if (T.chain && (T.evenOdd & 2) && nB < nSt) {
+                if ((order & 2) && nB < nSt) {
                     for (int c = 0; c < 2; ++c) {
                         for (int k = 2 * lane + c; k < nB; k += 2 * team)
-                            projectBendAt<COMP>(V, k, k, k + 1, invH2);
+                            projectBendAt<COMP>(V, k, k, k + 1);
                         teamSync(team, teamIdx);
                     }
-                } else if (T.chain && (T.evenOdd & 2)) {
+                } else if (order & 2) {
                     // with ghost frames, whose bends follow the real ones: one
                     // call for both, or the warp that holds a ghost runs the
                     // whole projection twice (a 64-segment cantilever's step:
@@ -1072,19 +1086,20 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                             const bool ghost = k >= nSt - 1;
                             const int a = ghost ? V.g->bA[k] : k;
                             const int b = ghost ? V.g->bB[k] : k + 1;
-                            projectBendAt<COMP>(V, k, a, b, invH2);
+                            projectBendAt<COMP>(V, k, a, b);
                         }
                         teamSync(team, teamIdx);
                     }
                 } else {
-                    for (int c = 0; c < T.bColors; ++c) {
+                    for (int c = 0; c < C.bColors; ++c) {
                         for (int ci = bCol[c] + lane; ci < bCol[c + 1]; ci += team)
-                            projectBendOne<COMP>(V, bOrder[ci], invH2);
+                            projectBendOne<COMP>(V, bOrder[ci]);
                         teamSync(team, teamIdx);
                     }
                 }
-                if (V.numPrims > 0 && maskNow != 0ull) {
-                    for (int i = lane; i < nP; i += team) projectSlots<COMP, FP64>(V, i, maskNow);
+                const unsigned long long mask = V.numPrims > 0 ? *primMask : 0ull;
+                if (mask != 0ull) {
+                    for (int i = lane; i < nP; i += team) projectSlots<COMP, FP64>(V, i, mask);
                     teamSync(team, teamIdx);
                 }
                 if (self) {
@@ -1101,9 +1116,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 
         // ---- per-step bookkeeping ----
         if (lane == 0) {
-            if (self) A.selfOverflow[r] += *S.overflow;
+            if (self) A.selfOverflow[C.rod] += *S.overflow;
             if (A.hold) {
-                DHold& H = A.hold[r];
+                DHold& H = A.hold[C.rod];
                 if (H.particle >= 0 && H.particle < nP) {
                     H.steps += 1;
                     if (A.holdInterval > 0 && H.steps % A.holdInterval == 0) {
@@ -1119,7 +1134,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     }  // steps of this launch
 
     // ---- stage out: bulk copies from shared memory, then the outputs ----
-    const DRod& out = A.rods[r];  // read again: not worth registers through the steps
+    const DRod& out = A.rods[C.rod];  // read again: not worth registers through the steps
     // every lane's writes above reach the async proxy before lane 0 copies
     fenceProxyAsyncShared();
     teamSync(team, teamIdx);
@@ -1142,9 +1157,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         for (int c = lane; c < live; c += team) A.selfPairs[out.poolOff + c] = S.pool[c].seg;
     }
     if (lane == 0) {
-        if (self) A.selfCount[r] = *S.live;
-        A.rodTime[r] = C.tRod;
-        if (C.wayP >= 0) A.waypoints[r].step = C.wayStep + stepsHere;
+        if (self) A.selfCount[C.rod] = *S.live;
+        A.rodTime[C.rod] = C.tRod;
+        if (C.wayP >= 0) A.waypoints[C.rod].step = C.wayStep + stepsHere;
     }
     // the stores have read the rows, and every lane's accesses of this shared
     // memory come before the next rod's bulk copies overwrite it
@@ -1161,7 +1176,6 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
                                                        int numGroups, int32_t* queue) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sGroup;
-    __shared__ int32_t queues[kMaxWarps][32];  // per warp: pairs that wait for the narrow phase
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) sGroup = atomicAdd(queue, 1);
@@ -1181,7 +1195,7 @@ __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* _
                                         Rk.hashTableSize, Rk.selfCapacity, 1, COMP ? 1 : 0, A.slotsShared)
                                   .bytes);
             }
-            runRod<COMP, FP64, SELF>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx, queues[tid >> 5]);
+            runRod<COMP, FP64, SELF>(A, A.work[first + teamIdx], smem + off, lane, team, teamIdx);
         }
         __syncthreads();
     }

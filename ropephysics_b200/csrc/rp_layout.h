@@ -68,7 +68,7 @@ struct RodLayout {
 //   batched kernel, whose teams may have 16 warps
 constexpr int32_t kMiscBytes = 320;
 constexpr int32_t kMiscBytesLong = 576;
-constexpr int32_t kContextBytes = 448;
+constexpr int32_t kContextBytes = 480;
 
 // Shared memory of one self contact while it is projected (batched kernel):
 // five 8-byte rows. A pool of nSt / 2 of them is the 20 nSt bytes that the
@@ -144,7 +144,7 @@ RP_HD inline RodLayout rodLayout(int32_t nP, int32_t nS, int32_t nSt, int32_t nB
         const int32_t most = 32 * kCompactBytes / 2;  // the smallest pool, 16 contacts
         const int32_t count = 16 * nSt + 32 * ((nSt + 7) / 8);
         L.centres = o;
-        L.blocks = o + 16 * nSt;
+        L.blocks = o + 16 * nSt;  // right behind the centres: the kernel counts on it
         o += count > most ? count : most;
         L.selfInt = o; o += nSt > 16 ? rpAlign16(8 * nSt) : 128;  // per-segment count and start
         L.hash = L.pool = L.levels = -1;

@@ -40,10 +40,10 @@ __device__ __forceinline__ RodView staticView(const DArgs& A, const DTemplate& T
     G.prims = A.prims + R.primOff;
     RodView V;
     V.numPrims = R.numPrims;
-    V.complianceScale = A.complianceScale[r];
-    V.frictionScale = A.frictionScale[r];
-    V.radius = R.radius;
-    V.contactMargin = R.contactMargin;
+    V.softness = A.invH2 * A.complianceScale[r];
+    G.frictionScale = A.frictionScale[r];
+    G.radius = R.radius;
+    G.contactMargin = R.contactMargin;
     return V;
 }
 
@@ -65,7 +65,7 @@ __device__ void buildSelfHashSerial(const RodView& V, const SelfScratch& S, int 
         const float len = norm(b - a);
         if (len > maxSegLen) maxSegLen = len;
     }
-    const float cell = maxSegLen + 2.0f * V.radius;
+    const float cell = maxSegLen + 2.0f * V.g->radius;
     *S.cellSize = cell;
     for (int t = 0; t <= table; ++t) S.cellStart[t] = 0;
     for (int j = 0; j < nSeg; ++j) {
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
     __syncthreads();
 
     const V3 g{A.gx, A.gy, A.gz};
-    const float h = A.h, invH2 = A.invH2;
+    const float h = A.h;
     const int interval = A.contactInterval;
     const int* sOrder = A.tOrder + T.sOrderOff;
     const int* bOrder = A.tOrder + T.bOrderOff;
@@ -253,12 +253,12 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
         for (int it = 0; it < A.iterations; ++it) {
             for (int c = 0; c < T.sColors; ++c) {
                 for (int ci = sCol[c] + tid; ci < sCol[c + 1]; ci += nth)
-                    projectStretchOne<COMP>(V, sOrder[ci], invH2);
+                    projectStretchOne<COMP>(V, sOrder[ci]);
                 __syncthreads();
             }
             for (int c = 0; c < T.bColors; ++c) {
                 for (int ci = bCol[c] + tid; ci < bCol[c + 1]; ci += nth)
-                    projectBendOne<COMP>(V, bOrder[ci], invH2);
+                    projectBendOne<COMP>(V, bOrder[ci]);
                 __syncthreads();
             }
             if (V.numPrims > 0) {

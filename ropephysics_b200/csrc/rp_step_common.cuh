@@ -42,6 +42,7 @@ struct RodGlobals {
     const float4* bComp;
     const float4* bRestD;
     const DPrim* prims;
+    float radius, contactMargin, frictionScale;
     // the rod's whole view, for the separately compiled fallbacks: a RodView
     // passed to them by reference would have to leave the registers
     const struct RodView* view;
@@ -62,10 +63,7 @@ struct RodView {
     DSlot* slots;
     const RodGlobals* g;  // loads, template data, primitives (global memory)
     int numPrims;
-    float complianceScale;
-    float frictionScale;
-    float radius;
-    float contactMargin;
+    float softness;  // per-rod compliance scale over h^2: alpha = compliance x softness
 };
 
 // Position update x[i] += a s. In reference order this is one fused
@@ -160,7 +158,7 @@ __device__ __forceinline__ void renormalizeFrameComp(const RodView& V, int j) {
 // operators: the fallback of projectStretchAt for what its shared
 // reciprocals do not cover. Not inlined, so that it costs the callers nothing.
 template <bool COMP>
-__device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int i0, int i1, int j, float invH2) {
+__device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int i0, int i1, int j) {
     const RodView& V = *g->view;
     const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
     const V3 iI = v3(V.g->invInertia[j]);
@@ -172,7 +170,7 @@ __device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int
     const V3 u = divs(rotateInv(q, d), l);
     const V3 C = u - V3{0.0f, 0.0f, 1.0f};
 
-    const V3 alpha = v3(sc) * (invH2 * V.complianceScale);
+    const V3 alpha = v3(sc) * V.softness;
     M3 A = madd(midentity((w0 + w1) / (l * l)), sandwichDiag<true>(mskew(u), iI));
     A.m[0][0] += alpha.x;
     A.m[1][1] += alpha.y;
@@ -207,7 +205,7 @@ __device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int
 // substeps x 3 sweeps, compensated, 194 -> 147 us; 4096 uneven rods, 50
 // substeps, self-collision on, 8.80 -> 7.77 ms.
 template <bool COMP>
-__device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0, int i1, int j, float invH2) {
+__device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0, int i1, int j) {
     const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
     const V3 iI = v3(V.g->invInertia[j]);
     if (w0 == 0.0f && w1 == 0.0f && norm2(iI) == 0.0f) return;
@@ -223,7 +221,7 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     const V3 u = rotateInv(q, d) * invL;
     const V3 C = u - V3{0.0f, 0.0f, 1.0f};
 
-    const V3 alpha = v3(sc) * (invH2 * V.complianceScale);
+    const V3 alpha = v3(sc) * V.softness;
     const Divisor dl = divisor(l, invL);
     const float ll = l * l;
     const float wl = quotient(w0 + w1, divisor(ll, recip(ll, ok)));
@@ -243,7 +241,7 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     const V3 theta = cwise(iI, cross(dL, u));
     const Q4 turned = COMP ? compRotationShared(theta * 0.5f, ok) : applyBodyDeltaShared(q, theta, ok);
     if (!ok) {
-        projectStretchPlain<COMP>(V.g, k, i0, i1, j, invH2);
+        projectStretchPlain<COMP>(V.g, k, i0, i1, j);
         return;
     }
     if (V.lamS) V.lamS[k] = f4(lam + dL);
@@ -258,15 +256,15 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
 }
 
 template <bool COMP>
-__device__ __forceinline__ void projectStretchOne(const RodView& V, int k, float invH2) {
-    projectStretchAt<COMP>(V, k, V.g->sP0[k], V.g->sP1[k], V.g->sSeg[k], invH2);
+__device__ __forceinline__ void projectStretchOne(const RodView& V, int k) {
+    projectStretchAt<COMP>(V, k, V.g->sP0[k], V.g->sP1[k], V.g->sSeg[k]);
 }
 
 // Bend/twist constraint k between frames a and b (bA[k], bB[k], or k, k+1
 // for a chain's real frames) with the plain operators: the fallback of
 // projectBendAt.
 template <bool COMP>
-__device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a, int b, float invH2) {
+__device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a, int b) {
     const RodView& V = *g0->view;
     const V3 iIa = v3(V.g->invInertia[a]), iIb = v3(V.g->invInertia[b]);
     const float4 bc = V.g->bComp[k];
@@ -280,7 +278,7 @@ __device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a
     const M3 Ja = mscale(madd(midentity(-p.w), skewPv), 1.0f / lbar);
     const M3 Jb = mscale(madd(midentity(p.w), skewPv), 1.0f / lbar);
 
-    const V3 alpha = v3(bc) * (invH2 * V.complianceScale);
+    const V3 alpha = v3(bc) * V.softness;
     M3 A = madd(sandwichDiag<false>(Ja, iIa), sandwichDiag<false>(Jb, iIb));
     A.m[0][0] += alpha.x;
     A.m[1][1] += alpha.y;
@@ -310,7 +308,7 @@ __device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a
 // The same projection, bit for bit, with shared reciprocals (see
 // projectStretchAt).
 template <bool COMP>
-__device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, int b, float invH2) {
+__device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, int b) {
     const V3 iIa = v3(V.g->invInertia[a]), iIb = v3(V.g->invInertia[b]);
     if (norm2(iIa) == 0.0f && norm2(iIb) == 0.0f) return;
 
@@ -327,7 +325,7 @@ __device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, in
     const M3 Ja = mscale(madd(midentity(-p.w), skewPv), invL);
     const M3 Jb = mscale(madd(midentity(p.w), skewPv), invL);
 
-    const V3 alpha = v3(bc) * (invH2 * V.complianceScale);
+    const V3 alpha = v3(bc) * V.softness;
     M3 A = madd(sandwichDiag<false>(Ja, iIa), sandwichDiag<false>(Jb, iIb));
     A.m[0][0] += alpha.x;
     A.m[1][1] += alpha.y;
@@ -342,7 +340,7 @@ __device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, in
     const Q4 ra = COMP ? compRotationShared(ta * 0.5f, ok) : applyBodyDeltaShared(qa, ta, ok);
     const Q4 rb = COMP ? compRotationShared(tb * 0.5f, ok) : applyBodyDeltaShared(qb, tb, ok);
     if (!ok) {
-        projectBendPlain<COMP>(V.g, k, a, b, invH2);
+        projectBendPlain<COMP>(V.g, k, a, b);
         return;
     }
     if (V.lamB) V.lamB[k] = f4(lam + dL);
@@ -361,8 +359,8 @@ __device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, in
 }
 
 template <bool COMP>
-__device__ __forceinline__ void projectBendOne(const RodView& V, int k, float invH2) {
-    projectBendAt<COMP>(V, k, V.g->bA[k], V.g->bB[k], invH2);
+__device__ __forceinline__ void projectBendOne(const RodView& V, int k) {
+    projectBendAt<COMP>(V, k, V.g->bA[k], V.g->bB[k]);
 }
 
 // ---------------------------------------------------------------- world contacts
@@ -378,21 +376,21 @@ __device__ __forceinline__ void generateSlot(const RodView& V, int i, const Prim
     V3 n;
     if (!COMP) {
         const V3 x = v3(V.x[i]);
-        const float gap = signedDistance(P, x, n) - V.radius;
-        if (gap >= V.contactMargin) return;
+        const float gap = signedDistance(P, x, n) - V.g->radius;
+        if (gap >= V.g->contactMargin) return;
         c.offset = dot(x, n) - gap;
     } else {
         const float4 xs = V.x[i], cs = V.xComp[i];
         const D3 xt{double(xs.x) - double(cs.x), double(xs.y) - double(cs.y), double(xs.z) - double(cs.z)};
-        const double gap = signedDistanceD(P, xt, n) - double(V.radius);
-        if (gap >= double(V.contactMargin)) return;
+        const double gap = signedDistanceD(P, xt, n) - double(V.g->radius);
+        if (gap >= double(V.g->contactMargin)) return;
         c.offset = float(gap);
     }
     c.state = 1;
     c.nx = n.x;
     c.ny = n.y;
     c.nz = n.z;
-    c.friction = P.friction * V.frictionScale;
+    c.friction = P.friction * V.g->frictionScale;
 }
 
 // A kept slot between regenerations: its multipliers restart. Compensated,
@@ -436,7 +434,7 @@ __device__ __forceinline__ void generateSlots(const RodView& V, int i, bool rege
 __device__ __forceinline__ unsigned long long primitivesNearBox(const RodView& V, V3 lo, V3 hi, int wl) {
     const V3 c = (lo + hi) * 0.5f;
     const V3 e = (hi - lo) * 0.5f;
-    const float reach = V.radius + V.contactMargin;
+    const float reach = V.g->radius + V.g->contactMargin;
     const float slack = 1e-3f * fabsf(reach) + 1e-4f +
                         1e-5f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + e.x + e.y + e.z);
     unsigned long long mask = 0ull;
@@ -610,7 +608,7 @@ __device__ __forceinline__ void writeSelfEntry(const RodView& V, DSelf& c, int j
     for (int m = 0; m < 4; ++m)
         dotSum = fma3(c.weight[m], dot(v3(V.x[c.idx[m]]), n), dotSum);
     c.offset = dotSum - separation;
-    c.friction = selfFriction * V.frictionScale;
+    c.friction = selfFriction * V.g->frictionScale;
     c.lambdaN = 0.0f;
     c.applied = 0.0f;
     c.seg = (j << 16) | k;
@@ -637,7 +635,7 @@ __device__ __forceinline__ void querySelfSegment(const RodView& V, const SelfScr
         const V3 cj = v3(cj4);
         const int cx = cellCoord(cj.x, cell), cy = cellCoord(cj.y, cell), cz = cellCoord(cj.z, cell);
         const V3 a0 = v3(V.x[V.g->sP0[j]]), a1 = v3(V.x[V.g->sP1[j]]);
-        const float twoR = 2.0f * V.radius;
+        const float twoR = 2.0f * V.g->radius;
         const float scaleSlack = 1e-6f * (1.0f + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z));
         for (int dz = -1; dz <= 1; ++dz)
             for (int dy = -1; dy <= 1; ++dy)
