@@ -66,6 +66,15 @@ __device__ __forceinline__ float warpMin(float f) {
     return r;
 }
 
+// A pointer into the kernel's shared memory, as one derived from the array
+// itself: only through such does the compiler use shared-memory instructions
+// (a pointer read back from memory is generic).
+template <typename T>
+__device__ __forceinline__ T* sharedMemory(T* p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    return reinterpret_cast<T*>(smem + (reinterpret_cast<const unsigned char*>(p) - smem));
+}
+
 __device__ __forceinline__ float4 driveVelocityB(const DDrive& d, double t) {
     const double s = double(d.amplitude) * double(d.omega) * cos(double(d.omega) * t + double(d.phase));
     return make_float4(float(s * double(d.ax)), float(s * double(d.ay)), float(s * double(d.az)), 0.0f);
@@ -163,6 +172,7 @@ struct TeamCtx {
     const int* sCol;
     const int* bCol;
     int32_t rod;                    // its index
+    int32_t chain;                  // segment j joins particles j and j + 1
     int32_t sColors, bColors;
     int32_t nP, nSt;
     int32_t table, selfGap, selfCapacity;
@@ -172,12 +182,21 @@ struct TeamCtx {
     int32_t stageFailed;            // a lane gave up waiting for the staged state
     uint64_t bar;                   // mbarrier of the rod's bulk stage-in
 
+    // the particles of segments j and k
+    __device__ void particles(int j, int k, int (&at)[4]) const {
+        at[0] = chain ? j : G.sP0[j];
+        at[1] = chain ? j + 1 : G.sP1[j];
+        at[2] = chain ? k : G.sP0[k];
+        at[3] = chain ? k + 1 : G.sP1[k];
+    }
     // the rod's misc words (rp_layout.h)
     __device__ int32_t* misc() const { return S.live - 1; }
     __device__ int32_t* numLevels() const { return misc() + 3; }  // projection levels of the pool
     __device__ int32_t* partial() const { return misc() + 16; }   // scan partials, one per warp
     __device__ int32_t* touching() const { return misc() + 14; }  // a self-contact pair touches this substep
     __device__ int32_t* numPairs() const { return misc() + 15; }  // how many do
+    // pair of every pool entry, (j << 16) | k, where the count's block bounds were
+    __device__ int32_t* ids() const { return reinterpret_cast<int32_t*>(sharedMemory(S.blocks)); }
     // behind the rod's hash in global memory (DRod::hashOff)
     __device__ int32_t* cursor() const { return S.cellStart + (table + 1); }  // placement cursors
     __device__ int32_t* lvlOrder() const { return cursor() + (table + 1); }   // coloured mode only
@@ -211,10 +230,11 @@ struct TeamCtx {
 // pool is built from the hash). Not inlined: few pairs get here, and its
 // body is shared by every caller.
 __device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float cell) {
-    const RodView& V = C.V;
     const SelfScratch& S = C.S;
-    const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                        v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
+    const float4* const x = sharedMemory(C.V.x);
+    int p[4];
+    C.particles(j, k, p);
+    const SegPair P = segmentPairNarrow(v3(x[p[0]]), v3(x[p[1]]), v3(x[p[2]]), v3(x[p[3]]), 2.0f * C.G.radius);
     if (P.separation >= 0.0f) return;
     const unsigned cells = bucketCells(S.centres[j], S.centres[k], cell, C.table);
     if (cells) {
@@ -374,17 +394,22 @@ __device__ __forceinline__ void orderPool(const TeamCtx& C, int live, int precis
     constexpr unsigned kAll = 0xffffffffu;
     const SelfScratch& S = C.S;
     const int nP = C.nP;
-    int32_t* const last = reinterpret_cast<int32_t*>(S.centres);   // per particle: its highest level + 1
+    int32_t* const last = reinterpret_cast<int32_t*>(sharedMemory(S.centres));  // per particle: its highest level + 1
     int32_t* const lanes = last + nP;                              // per particle: this chunk's lanes
-    int32_t* const place = S.segCount;
+    int32_t* const place = sharedMemory(S.segCount);
+    const int32_t* const ids = C.ids();
+    auto particles = [&](int c) {
+        const int j = ids[c] >> 16, k = ids[c] & 0xffff;
+        return C.chain ? make_int4(j, j + 1, k, k + 1) : *reinterpret_cast<const int4*>(S.pool[c].idx);
+    };
     int kept = live;
     for (int c0 = 0; c0 < live; c0 += 32) {
         const int c = c0 + lane;
         bool ok = true;
         if (c < live) {
-            const int4 at = *reinterpret_cast<const int4*>(S.pool[c].idx);
+            const int4 at = particles(c);
             ok = min(min(at.x, at.y), min(at.z, at.w)) >= 0 && max(max(at.x, at.y), max(at.z, at.w)) < nP &&
-                 S.pool[c].seg != -1;
+                 ids[c] != -1;
             if (ok) {
                 last[at.x] = last[at.y] = last[at.z] = last[at.w] = 0;
                 lanes[at.x] = lanes[at.y] = lanes[at.z] = lanes[at.w] = 0;
@@ -424,7 +449,7 @@ __device__ __forceinline__ void orderPool(const TeamCtx& C, int live, int precis
         int4 at = make_int4(0, 0, 0, 0);
         int level = 0;
         if (mine) {
-            at = *reinterpret_cast<const int4*>(S.pool[c].idx);
+            at = particles(c);
             level = max(max(last[at.x], last[at.y]), max(last[at.z], last[at.w]));
             atomicOr(&lanes[at.x], 1 << lane);
             atomicOr(&lanes[at.y], 1 << lane);
@@ -540,8 +565,10 @@ __device__ __forceinline__ void fillSelfPool(const TeamCtx& C, float cell, int l
 // S.segStart[0..numPairs), numPairs <= 32, with the cells in S.sorted; S.segCount
 // holds the pairs' cells afterwards.
 __device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int lane) {
-    const RodView& V = C.V;
     const SelfScratch& S = C.S;
+    const float4* const x = sharedMemory(C.V.x);
+    const float friction = C.selfFriction * C.G.frictionScale;
+    int32_t* const ids = C.ids();
     const bool mine = lane < numPairs;
     int j = 0, k = 0;
     unsigned cells = 0u;
@@ -556,8 +583,9 @@ __device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int
     if (mine) S.segCount[lane] = int32_t(cells);
     __syncwarp();
     if (mine) {
-        const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
+        int at[4];
+        C.particles(j, k, at);
+        const SegPair P = segmentPairNarrow(v3(x[at[0]]), v3(x[at[1]]), v3(x[at[2]]), v3(x[at[3]]), 2.0f * C.G.radius);
         // entries of the pairs of earlier segments
         int before = 0;
         for (int q = 0; q < numPairs; ++q)
@@ -572,7 +600,10 @@ __device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int
                 const unsigned cq = unsigned(S.segCount[q]);
                 rank += __popc(cq & below) + (((cq >> t) & 1u) && (pq & 0xffff) < k ? 1 : 0);
             }
-            if (rank < C.selfCapacity) writeSelfEntry(V, S.pool[rank], j, k, P, C.selfFriction);
+            if (rank < C.selfCapacity) {
+                writeSelfEntryAt(x, S.pool[rank], at, j, k, P, friction);
+                ids[rank] = (j << 16) | k;
+            }
         }
     }
     return total;
@@ -591,10 +622,12 @@ __device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int
 // substeps 8.53 -> 2.08 ms, and rods in free fall, which touch now and then,
 // 4096 of 16-512, 7.65 -> 6.93 ms.
 __device__ __forceinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs, int lane, int team, int teamIdx) {
-    const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const int nSt = C.nSt;
-    int32_t* const head = reinterpret_cast<int32_t*>(S.centres);  // per segment: its last linked pair
+    const float4* const x = sharedMemory(C.V.x);
+    const float friction = C.selfFriction * C.G.frictionScale;
+    int32_t* const ids = C.ids();
+    int32_t* const head = reinterpret_cast<int32_t*>(sharedMemory(S.centres));  // per segment: its last linked pair
     int32_t* const next = head + nSt;                             // per pair
     int32_t* const cellsOf = next + nSt;                          // per pair
     for (int p = lane; p < numPairs; p += team) {
@@ -609,8 +642,9 @@ __device__ __forceinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs,
         const int before = S.segCount[j];
         if (before >= C.selfCapacity) continue;
         const unsigned cells = unsigned(cellsOf[p]);
-        const SegPair P = segmentPairNarrow(v3(V.x[V.g->sP0[j]]), v3(V.x[V.g->sP1[j]]), v3(V.x[V.g->sP0[k]]),
-                                            v3(V.x[V.g->sP1[k]]), 2.0f * V.g->radius);
+        int at[4];
+        C.particles(j, k, at);
+        const SegPair P = segmentPairNarrow(v3(x[at[0]]), v3(x[at[1]]), v3(x[at[2]]), v3(x[at[3]]), 2.0f * C.G.radius);
         for (unsigned rest = cells; rest; rest &= rest - 1u) {
             const int t = __ffs(rest) - 1;
             const unsigned below = (1u << t) - 1u;
@@ -619,7 +653,10 @@ __device__ __forceinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs,
                 const unsigned cq = unsigned(cellsOf[q]);
                 rank += __popc(cq & below) + (((cq >> t) & 1u) && (S.segStart[q] & 0xffff) < k ? 1 : 0);
             }
-            if (rank < C.selfCapacity) writeSelfEntry(V, S.pool[rank], j, k, P, C.selfFriction);
+            if (rank < C.selfCapacity) {
+                writeSelfEntryAt(x, S.pool[rank], at, j, k, P, friction);
+                ids[rank] = (j << 16) | k;
+            }
         }
     }
     return total;
@@ -642,6 +679,8 @@ __device__ __noinline__ void buildPool(const TeamCtx& C, float cell, int precisi
         teamSync(team, teamIdx);
         total = teamExclusiveScan(S.segStart, nSt, lane, team, teamIdx, C.partial());
         fillSelfPool(C, cell, min(total, C.selfCapacity), lane, team, teamIdx);
+        teamSync(team, teamIdx);
+        for (int c = lane; c < min(total, C.selfCapacity); c += team) C.ids()[c] = S.pool[c].seg;
     }
     if (lane == 0) {
         *S.live = min(total, C.selfCapacity);
@@ -822,6 +861,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         C.sColors = T.sColors;
         C.bColors = T.bColors;
         C.rod = r;
+        C.chain = T.chain;
         *numLevels = 0;
         *primMask = ~0ull;
         // simulated time of this rod, advanced per step exactly as the

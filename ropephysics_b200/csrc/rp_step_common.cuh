@@ -588,30 +588,32 @@ static __device__ __noinline__ SegPair segmentPairNarrow(V3 a0, V3 a1, V3 b0, V3
 // The pool entry of touching segments j < k from their narrow phase P: the
 // contact normal, the four particles and their weights, the offset from the
 // current positions, friction, zeroed multipliers and the pair id.
-__device__ __forceinline__ void writeSelfEntry(const RodView& V, DSelf& c, int j, int k, const SegPair& P,
-                                               float selfFriction) {
+__device__ __forceinline__ void writeSelfEntryAt(const float4* x, DSelf& c, const int (&at)[4], int j, int k,
+                                                 const SegPair& P, float friction) {
     const float u = P.u, w = P.w, dist = P.dist, separation = P.separation;
     const V3 delta = P.delta;
     const V3 n = dist > 1e-12f ? divs(delta, dist) : V3{0.0f, 0.0f, 1.0f};
     c.nx = n.x;
     c.ny = n.y;
     c.nz = n.z;
-    c.idx[0] = V.g->sP0[j];
-    c.idx[1] = V.g->sP1[j];
-    c.idx[2] = V.g->sP0[k];
-    c.idx[3] = V.g->sP1[k];
-    c.weight[0] = 1.0f - u;
-    c.weight[1] = u;
-    c.weight[2] = -(1.0f - w);
-    c.weight[3] = -w;
+    const float weight[4] = {1.0f - u, u, -(1.0f - w), -w};
     float dotSum = 0.0f;
-    for (int m = 0; m < 4; ++m)
-        dotSum = fma3(c.weight[m], dot(v3(V.x[c.idx[m]]), n), dotSum);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        c.idx[m] = at[m];
+        c.weight[m] = weight[m];
+        dotSum = fma3(weight[m], dot(v3(x[at[m]]), n), dotSum);
+    }
     c.offset = dotSum - separation;
-    c.friction = selfFriction * V.g->frictionScale;
+    c.friction = friction;
     c.lambdaN = 0.0f;
     c.applied = 0.0f;
     c.seg = (j << 16) | k;
+}
+__device__ __forceinline__ void writeSelfEntry(const RodView& V, DSelf& c, int j, int k, const SegPair& P,
+                                               float selfFriction) {
+    const int at[4] = {V.g->sP0[j], V.g->sP1[j], V.g->sP0[k], V.g->sP1[k]};
+    writeSelfEntryAt(V.x, c, at, j, k, P, selfFriction * V.g->frictionScale);
 }
 
 // Contacts of segment j with later segments, in the reference's candidate
