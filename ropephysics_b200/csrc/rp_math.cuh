@@ -207,6 +207,21 @@ __device__ __forceinline__ M3 sandwichDiag(const M3& A, V3 d) {
     }
     return r;
 }
+// The lower triangle of s I + sandwichDiag<true>(mskew(v), d) by its nonzero
+// terms: for finite v and d the products with the zero diagonal only add
+// zeros, and s I or the sum's leading +0 absorbs their sign. (Not finite:
+// the solve refuses it.) 15 operations instead of 27, 1 % of a step.
+__device__ __forceinline__ M3 skewSandwichPlus(float s, V3 v, V3 d) {
+    const float zx = v.z * d.x, zy = -v.z * d.y, yz = v.y * d.z, xz = -v.x * d.z, yx = -v.y * d.x, xy = v.x * d.y;
+    M3 r = mzero();
+    r.m[0][0] = s + fma3(yz, v.y, zy * -v.z);
+    r.m[1][0] = 0.0f + xz * v.y;
+    r.m[1][1] = s + fma3(xz, -v.x, zx * v.z);
+    r.m[2][0] = 0.0f + xy * -v.z;
+    r.m[2][1] = 0.0f + yx * v.z;
+    r.m[2][2] = s + fma3(xy, v.x, yx * -v.y);
+    return r;
+}
 // Symmetric positive-definite 3x3 solve by Cholesky; false if not SPD.
 __device__ __forceinline__ bool solveSPD3(const M3& A, V3 b, V3& y) {
     float l00 = A.m[0][0];

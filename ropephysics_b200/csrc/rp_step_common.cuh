@@ -227,7 +227,7 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     const float wl = quotient(w0 + w1, divisor(ll, recip(ll, ok)));
     const float s0 = quotient(w0, dl), s1 = quotient(w1, dl);
     ok = ok & (fmaxf(fabsf(w0), fabsf(w1)) <= 0x1p60f);
-    M3 A = madd(midentity(wl), sandwichDiag<true>(mskew(u), iI));
+    M3 A = skewSandwichPlus(wl, u, iI);
     A.m[0][0] += alpha.x;
     A.m[1][1] += alpha.y;
     A.m[2][2] += alpha.z;
