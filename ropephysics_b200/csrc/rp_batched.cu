@@ -737,12 +737,10 @@ __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, in
                 const unsigned a = __float_as_uint(i.x), b = __float_as_uint(i.y);
                 const int at[4] = {int(a & 0xffffu), int(a >> 16), int(b & 0xffffu), int(b >> 16)};
                 const float weight[4] = {1.0f - uw.x, uw.x, -(1.0f - uw.y), -uw.y};
-                const float im[4] = {V.g->invMass[at[0]], V.g->invMass[at[1]], V.g->invMass[at[2]],
-                                     V.g->invMass[at[3]]};
                 const V3 n{nxy.x, nxy.y, nzo.x};
                 const bool distinct = at[0] != at[1] && at[0] != at[2] && at[0] != at[3] && at[1] != at[2] &&
                                       at[1] != at[3] && at[2] != at[3];
-                if (!distinct || !projectSelfDistinct<COMP>(x, xPrev, xComp, at, weight, im, n, nzo.y, friction,
+                if (!distinct || !projectSelfDistinct<COMP>(x, xPrev, xComp, at, weight, n, nzo.y, friction,
                                                             lam.x, lam.y)) {
                     DSelf k;
                     for (int m = 0; m < 4; ++m) {
@@ -1078,9 +1076,12 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
             // velocities pass from the update to the prediction in registers;
             // the prediction's own velocity is never read (the next update
             // replaces it), so velocities are in memory only between steps
+            // (the inverse mass travels in xPrev's fourth word: read from global
+            // memory once a step)
             for (int i = lane; i < nP; i += team) {
-                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, h, A.linDecay) : C.velocity[i];
-                predictParticleFrom<COMP>(V, i, h, g, vi, nullptr);
+                const float w = sub > 0 ? V.xPrev[i].w : V.g->invMass[i];
+                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, w, h, A.linDecay) : C.velocity[i];
+                predictParticleFrom<COMP>(V, i, w, h, g, vi, nullptr);
             }
             for (int j = lane; j < nS; j += team) {
                 const float4 wj = sub > 0 ? finishedOmega<COMP>(V, j, h, A.angDecay) : C.omega[j];
@@ -1150,7 +1151,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 
         }
         // the step's last velocity update
-        for (int i = lane; i < nP; i += team) C.velocity[i] = finishedVelocity<COMP>(V, i, h, A.linDecay);
+        for (int i = lane; i < nP; i += team) C.velocity[i] = finishedVelocity<COMP>(V, i, V.xPrev[i].w, h, A.linDecay);
         for (int j = lane; j < nS; j += team) C.omega[j] = finishedOmega<COMP>(V, j, h, A.angDecay);
         teamSync(team, teamIdx);
 

@@ -40,7 +40,7 @@ struct M3 {
 
 __device__ __forceinline__ V3 v3(float x, float y, float z) { return V3{x, y, z}; }
 __device__ __forceinline__ V3 v3(float4 a) { return V3{a.x, a.y, a.z}; }
-__device__ __forceinline__ float4 f4(V3 a) { return make_float4(a.x, a.y, a.z, 0.0f); }
+__device__ __forceinline__ float4 f4(V3 a, float w = 0.0f) { return make_float4(a.x, a.y, a.z, w); }
 __device__ __forceinline__ Q4 q4(float4 a) { return Q4{a.x, a.y, a.z, a.w}; }
 __device__ __forceinline__ float4 f4(Q4 q) { return make_float4(q.w, q.x, q.y, q.z); }
 

@@ -51,7 +51,7 @@ struct RodGlobals {
 struct RodView {
     // dynamic state (shared or global memory)
     float4* x;
-    float4* xPrev;
+    float4* xPrev;  // w: the particle's inverse mass, from the prediction on
     float4* v;
     float4* q;
     float4* qPrev;
@@ -87,7 +87,8 @@ __device__ __forceinline__ void addPos(const RodView& V, int i, V3 a, float s) {
         const V3 c = (t - v3(xs)) - y;
         V.x[i] = f4(t);
         V.xComp[i] = f4(c);
-        V.xPrev[i] = f4(v3(V.xPrev[i]) + d);
+        const float4 xp = V.xPrev[i];
+        V.xPrev[i] = f4(v3(xp) + d, xp.w);
     }
 }
 
@@ -497,7 +498,7 @@ __device__ __forceinline__ void generateSlotsMasked(const RodView& V, int i, boo
 // double-precision cone test (RP_PRECISION_FP64_CONE).
 template <bool COMP, bool FP64>
 __device__ __forceinline__ void projectSlots(const RodView& V, int i, unsigned long long mask) {
-    const float w = V.g->invMass[i];
+    const float w = V.xPrev[i].w;
     if (w <= 0.0f) return;
     const int base = i * V.numPrims;
     for (int k = 0; k < V.numPrims; ++k) {
@@ -703,30 +704,31 @@ __device__ __forceinline__ int buildProjectionColors(const DSelf* pool, int live
 }
 
 // The four-particle case of the contact projection on distinct particles,
-// with everything read before anything is written: the reads of positions,
-// displacements and masses overlap, where projectSelf waits for each
+// with everything read before anything is written: the reads of positions
+// and displacements (with the masses) overlap, where projectSelf waits for each
 // particle's store before it reads the next. `lambdaN` and `applied` are the
 // contact's multipliers, updated in place. Returns false, having written
 // nothing, for what the shared reciprocals do not cover (projectSelf does it).
 template <bool COMP>
 __device__ __forceinline__ bool projectSelfDistinct(float4* x, float4* xPrev, float4* xComp, const int (&at)[4],
-                                                    const float (&weight)[4], const float (&im)[4], V3 n,
-                                                    float offset, float friction, float& lambdaN,
+                                                    const float (&weight)[4], V3 n, float offset, float friction, float& lambdaN,
                                                     float& applied) {
-    float wEff = 0.0f;
+    float wEff = 0.0f, im[4];
+    V3 p[4], c[4], d[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const float4 xp = xPrev[at[m]];
+        d[m] = v3(xp);
+        im[m] = xp.w;
+        p[m] = v3(x[at[m]]);
+        if (COMP) c[m] = v3(xComp[at[m]]);
+    }
 #pragma unroll
     for (int m = 0; m < 4; ++m) wEff = fma3(weight[m] * weight[m], im[m], wEff);
     if (wEff <= 0.0f) return true;
     bool ok = true;
     const Divisor dw = divisor(wEff, recip(wEff, ok));
     ok = ok & (fmaxf(fmaxf(im[0], im[1]), fmaxf(im[2], im[3])) <= 0x1p60f);
-    V3 p[4], c[4], d[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        p[m] = v3(x[at[m]]);
-        d[m] = v3(xPrev[at[m]]);
-        if (COMP) c[m] = v3(xComp[at[m]]);
-    }
     // addPos on the values held here
     auto add = [&](int m, V3 a, float s) {
         if (!COMP) {
@@ -784,7 +786,7 @@ __device__ __forceinline__ bool projectSelfDistinct(float4* x, float4* xPrev, fl
         x[at[m]] = f4(p[m]);
         if (COMP) {
             xComp[at[m]] = f4(c[m]);
-            xPrev[at[m]] = f4(d[m]);
+            xPrev[at[m]] = f4(d[m], im[m]);
         }
     }
     return true;
@@ -829,15 +831,14 @@ __device__ __forceinline__ void projectSelf(const RodView& V, DSelf& c) {
 
 // ---------------------------------------------------------------- predict / finish
 
-// Prediction of particle i from the velocity vIn. The predicted velocity is
+// Prediction of particle i, of inverse mass w, from the velocity vIn. The predicted velocity is
 // written to *vOut when it is given: the plain kernel keeps it in its state
 // array; the batched kernel drops it, because the substep's velocity update
 // replaces it without reading it.
 template <bool COMP>
-__device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, float h, V3 g, float4 vIn,
+__device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, float w, float h, V3 g, float4 vIn,
                                                     float4* vOut) {
-    V.xPrev[i] = COMP ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : V.x[i];
-    const float w = V.g->invMass[i];
+    V.xPrev[i] = COMP ? make_float4(0.0f, 0.0f, 0.0f, w) : f4(v3(V.x[i]), w);
     if (w == 0.0f) {
         addPos<COMP>(V, i, v3(V.g->kin[i]), h);  // prescribed motion
         return;
@@ -849,7 +850,7 @@ __device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, flo
 
 template <bool COMP>
 __device__ __forceinline__ void predictParticle(const RodView& V, int i, float h, V3 g) {
-    predictParticleFrom<COMP>(V, i, h, g, V.v[i], &V.v[i]);
+    predictParticleFrom<COMP>(V, i, V.g->invMass[i], h, g, V.v[i], &V.v[i]);
 }
 
 // Prediction of frame j from the angular velocity wIn (*wOut as for the
@@ -889,15 +890,15 @@ __device__ __forceinline__ void predictFrame(const RodView& V, int j, float h) {
 // Velocity of particle i at the end of a substep (recovered from its
 // displacement; a kinematic particle takes its prescribed velocity).
 template <bool COMP>
-__device__ __forceinline__ float4 finishedVelocity(const RodView& V, int i, float h, float linDecay) {
-    if (V.g->invMass[i] == 0.0f) return V.g->kin[i];
+__device__ __forceinline__ float4 finishedVelocity(const RodView& V, int i, float w, float h, float linDecay) {
+    if (w == 0.0f) return V.g->kin[i];
     const V3 d = dispOf<COMP>(V, i);
     return f4(divs(d, h) * linDecay);
 }
 
 template <bool COMP>
 __device__ __forceinline__ void finishParticle(const RodView& V, int i, float h, float linDecay) {
-    V.v[i] = finishedVelocity<COMP>(V, i, h, linDecay);
+    V.v[i] = finishedVelocity<COMP>(V, i, V.xPrev[i].w, h, linDecay);
 }
 
 // Angular velocity of frame j at the end of a substep (from the substep's
