@@ -786,6 +786,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
     RodView V;
     V.g = &C.G;
     V.numPrims = R.numPrims;
+    V.rowMask = T.evenOdd & 4 ? 0 : -1;
     V.softness = A.invH2 * A.complianceScale[r];
     V.q = reinterpret_cast<float4*>(base + L.q);
     V.qPrev = COMP ? A.gqPrev + R.sOff : reinterpret_cast<float4*>(base + L.qPrev);

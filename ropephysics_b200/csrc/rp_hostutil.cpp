@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -192,6 +193,12 @@ void makeTemplate(const rp_rod_desc* d, TemplateHost& h) {
                          std::vector<int>(h.colorStart.begin() + T.bColorOff, h.colorStart.end()), d->num_bend)
                      ? 2
                      : 0);
+    auto same = [](const std::vector<float4>& v) {
+        for (const float4& a : v)
+            if (std::memcmp(&a, &v[0], sizeof(float4)) != 0) return false;
+        return true;
+    };
+    if (same(h.invInertia) && same(h.inertia) && same(h.sComp) && same(h.bComp) && same(h.bRestD)) T.evenOdd |= 4;
 }
 
 namespace {

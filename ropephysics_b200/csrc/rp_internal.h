@@ -36,7 +36,9 @@ struct DTemplate {
     int32_t chain;                 // 1: stretch k = (k, k+1, frame k) for all k, bends of
                                    // real frames (k, k+1) for k < nSt-1, ghosts after
     int32_t evenOdd;               // bit 0: stretch colour order is {0,2,4..},{1,3,5..};
-                                   // bit 1: the same for the bends
+                                   // bit 1: the same for the bends; bit 2: every frame,
+                                   // stretch and bend has the same inertia, compliance and
+                                   // rest data, bit for bit
 };
 
 // One rod of the batch.

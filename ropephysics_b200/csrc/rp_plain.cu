@@ -40,6 +40,7 @@ __device__ __forceinline__ RodView staticView(const DArgs& A, const DTemplate& T
     G.prims = A.prims + R.primOff;
     RodView V;
     V.numPrims = R.numPrims;
+    V.rowMask = T.evenOdd & 4 ? 0 : -1;
     V.softness = A.invH2 * A.complianceScale[r];
     G.frictionScale = A.frictionScale[r];
     G.radius = R.radius;
