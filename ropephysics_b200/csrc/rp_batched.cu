@@ -910,6 +910,10 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         return;
     }
 
+    // the inverse masses ride in the positions' fourth word: every phase that
+    // needs one reads the position anyway
+    for (int i = lane; i < nP; i += team) V.x[i].w = V.g->invMass[i];
+
     const V3 g{A.gx, A.gy, A.gz};
     const float h = A.h;
     const int interval = A.contactInterval;
@@ -1077,12 +1081,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
             // velocities pass from the update to the prediction in registers;
             // the prediction's own velocity is never read (the next update
             // replaces it), so velocities are in memory only between steps
-            // (the inverse mass travels in xPrev's fourth word: read from global
-            // memory once a step)
             for (int i = lane; i < nP; i += team) {
-                const float w = sub > 0 ? V.xPrev[i].w : V.g->invMass[i];
-                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, w, h, A.linDecay) : C.velocity[i];
-                predictParticleFrom<COMP>(V, i, w, h, g, vi, nullptr);
+                const float4 vi = sub > 0 ? finishedVelocity<COMP>(V, i, h, A.linDecay) : C.velocity[i];
+                predictParticleFrom<COMP>(V, i, h, g, vi, nullptr);
             }
             for (int j = lane; j < nS; j += team) {
                 const float4 wj = sub > 0 ? finishedOmega<COMP>(V, j, h, A.angDecay) : C.omega[j];
@@ -1152,7 +1153,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 
         }
         // the step's last velocity update
-        for (int i = lane; i < nP; i += team) C.velocity[i] = finishedVelocity<COMP>(V, i, V.xPrev[i].w, h, A.linDecay);
+        for (int i = lane; i < nP; i += team) C.velocity[i] = finishedVelocity<COMP>(V, i, h, A.linDecay);
         for (int j = lane; j < nS; j += team) C.omega[j] = finishedOmega<COMP>(V, j, h, A.angDecay);
         teamSync(team, teamIdx);
 
@@ -1177,6 +1178,7 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 
     // ---- stage out: bulk copies from shared memory, then the outputs ----
     const DRod& out = A.rods[C.rod];  // read again: not worth registers through the steps
+    for (int i = lane; i < nP; i += team) V.x[i].w = 0.0f;  // the rows' pad in global memory
     // every lane's writes above reach the async proxy before lane 0 copies
     fenceProxyAsyncShared();
     teamSync(team, teamIdx);

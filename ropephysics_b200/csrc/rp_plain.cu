@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
         const float4* gc = A.xComp + R.pOff;
         const float4* gt = A.torque + R.sOff;
         for (int i = tid; i < nP; i += nth) {
-            V.x[i] = gx[i];
+            V.x[i] = f4(v3(gx[i]), V.g->invMass[i]);  // the inverse mass in the fourth word
             V.v[i] = gv[i];
             G.force[i] = gf[i];
             G.kin[i] = i == driveP ? driveV : gk[i];
@@ -195,8 +195,9 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
             V.omega[j] = gw[j];
             G.torque[j] = gt[j];
         }
-    } else if (driveP >= 0 && tid == 0) {
-        G.kin[driveP] = driveV;
+    } else {
+        for (int i = tid; i < nP; i += nth) gx[i].w = V.g->invMass[i];
+        if (driveP >= 0 && tid == 0) G.kin[driveP] = driveV;
     }
     __syncthreads();
 
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
     if (!GMEM) {
         float4* gc = A.xComp + R.pOff;
         for (int i = tid; i < nP; i += nth) {
-            gx[i] = V.x[i];
+            gx[i] = f4(v3(V.x[i]));
             gv[i] = V.v[i];
             if (COMP) gc[i] = V.xComp[i];
         }
@@ -291,6 +292,8 @@ __global__ void __launch_bounds__(128, 4) kPlainStep(DArgs A) {
             gw[j] = V.omega[j];
         }
         if (driveP >= 0 && tid == 0) A.kinVel[R.pOff + driveP] = driveV;
+    } else {
+        for (int i = tid; i < nP; i += nth) gx[i].w = 0.0f;
     }
     if (V.numPrims > 0 && A.contactState) {
         const int slots = nP * V.numPrims;

@@ -50,8 +50,8 @@ struct RodGlobals {
 
 struct RodView {
     // dynamic state (shared or global memory)
-    float4* x;
-    float4* xPrev;  // w: the particle's inverse mass, from the prediction on
+    float4* x;      // w: the particle's inverse mass, while a kernel steps the rod
+    float4* xPrev;
     float4* v;
     float4* q;
     float4* qPrev;
@@ -83,7 +83,8 @@ struct RodView {
 template <bool COMP>
 __device__ __forceinline__ void addPos(const RodView& V, int i, V3 a, float s) {
     if (!COMP) {
-        V.x[i] = f4(fmav(a, s, v3(V.x[i])));
+        const float4 xs = V.x[i];
+        V.x[i] = f4(fmav(a, s, v3(xs)), xs.w);
     } else {
         const V3 d = a * s;
         const float4 xs = V.x[i];
@@ -91,10 +92,9 @@ __device__ __forceinline__ void addPos(const RodView& V, int i, V3 a, float s) {
         const V3 y = d - v3(cs);
         const V3 t = v3(xs) + y;
         const V3 c = (t - v3(xs)) - y;
-        V.x[i] = f4(t);
+        V.x[i] = f4(t, xs.w);
         V.xComp[i] = f4(c);
-        const float4 xp = V.xPrev[i];
-        V.xPrev[i] = f4(v3(xp) + d, xp.w);
+        V.xPrev[i] = f4(v3(V.xPrev[i]) + d);
     }
 }
 
@@ -213,7 +213,8 @@ __device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int
 // substeps, self-collision on, 8.80 -> 7.77 ms.
 template <bool COMP>
 __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0, int i1, int j) {
-    const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
+    const float4 x0 = V.x[i0], x1 = V.x[i1];
+    const float w0 = x0.w, w1 = x1.w;
     const V3 iI = v3(V.g->invInertia[j & V.rowMask]);
     if (w0 == 0.0f && w1 == 0.0f && norm2(iI) == 0.0f) return;
 
@@ -222,7 +223,7 @@ __device__ __forceinline__ void projectStretchAt(const RodView& V, int k, int i0
     const float l = sc.w;
     const float invL = recip(l, ok);
     const Q4 q = q4(V.q[j]);
-    V3 d = v3(V.x[i1]) - v3(V.x[i0]);
+    V3 d = v3(x1) - v3(x0);
     // compensated mode: the segment vector of the true (x - xComp) positions
     if (COMP) d = d - (v3(V.xComp[i1]) - v3(V.xComp[i0]));
     const V3 u = rotateInv(q, d) * invL;
@@ -415,7 +416,7 @@ __device__ __forceinline__ void keepSlot(const RodView& V, int i, DSlot& c) {
 template <bool COMP>
 __device__ __forceinline__ void generateSlots(const RodView& V, int i, bool regenerate) {
     const int base = i * V.numPrims;
-    const float w = V.g->invMass[i];
+    const float w = V.x[i].w;
     for (int k = 0; k < V.numPrims; ++k) {
         DSlot& c = V.slots[base + k];
         c.lambdaN = 0.0f;
@@ -483,7 +484,7 @@ template <bool COMP>
 __device__ __forceinline__ void generateSlotsMasked(const RodView& V, int i, bool regenerate,
                                                     unsigned long long mask) {
     const int base = i * V.numPrims;
-    const float w = V.g->invMass[i];
+    const float w = V.x[i].w;
     for (int k = 0; k < V.numPrims; ++k) {
         if (!((mask >> k) & 1ull)) continue;
         DSlot& c = V.slots[base + k];
@@ -504,7 +505,7 @@ __device__ __forceinline__ void generateSlotsMasked(const RodView& V, int i, boo
 // double-precision cone test (RP_PRECISION_FP64_CONE).
 template <bool COMP, bool FP64>
 __device__ __forceinline__ void projectSlots(const RodView& V, int i, unsigned long long mask) {
-    const float w = V.xPrev[i].w;
+    const float w = V.x[i].w;
     if (w <= 0.0f) return;
     const int base = i * V.numPrims;
     for (int k = 0; k < V.numPrims; ++k) {
@@ -711,7 +712,7 @@ __device__ __forceinline__ int buildProjectionColors(const DSelf* pool, int live
 
 // The four-particle case of the contact projection on distinct particles,
 // with everything read before anything is written: the reads of positions
-// and displacements (with the masses) overlap, where projectSelf waits for each
+// (with the masses) and displacements overlap, where projectSelf waits for each
 // particle's store before it reads the next. `lambdaN` and `applied` are the
 // contact's multipliers, updated in place. Returns false, having written
 // nothing, for what the shared reciprocals do not cover (projectSelf does it).
@@ -723,10 +724,10 @@ __device__ __forceinline__ bool projectSelfDistinct(float4* x, float4* xPrev, fl
     V3 p[4], c[4], d[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        const float4 xp = xPrev[at[m]];
-        d[m] = v3(xp);
-        im[m] = xp.w;
-        p[m] = v3(x[at[m]]);
+        const float4 xs = x[at[m]];
+        p[m] = v3(xs);
+        im[m] = xs.w;
+        d[m] = v3(xPrev[at[m]]);
         if (COMP) c[m] = v3(xComp[at[m]]);
     }
 #pragma unroll
@@ -789,10 +790,10 @@ __device__ __forceinline__ bool projectSelfDistinct(float4* x, float4* xPrev, fl
     applied = rubbed;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        x[at[m]] = f4(p[m]);
+        x[at[m]] = f4(p[m], im[m]);
         if (COMP) {
             xComp[at[m]] = f4(c[m]);
-            xPrev[at[m]] = f4(d[m], im[m]);
+            xPrev[at[m]] = f4(d[m]);
         }
     }
     return true;
@@ -837,14 +838,16 @@ __device__ __forceinline__ void projectSelf(const RodView& V, DSelf& c) {
 
 // ---------------------------------------------------------------- predict / finish
 
-// Prediction of particle i, of inverse mass w, from the velocity vIn. The predicted velocity is
+// Prediction of particle i from the velocity vIn. The predicted velocity is
 // written to *vOut when it is given: the plain kernel keeps it in its state
 // array; the batched kernel drops it, because the substep's velocity update
 // replaces it without reading it.
 template <bool COMP>
-__device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, float w, float h, V3 g, float4 vIn,
+__device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, float h, V3 g, float4 vIn,
                                                     float4* vOut) {
-    V.xPrev[i] = COMP ? make_float4(0.0f, 0.0f, 0.0f, w) : f4(v3(V.x[i]), w);
+    const float4 xs = V.x[i];
+    const float w = xs.w;
+    V.xPrev[i] = COMP ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : xs;
     if (w == 0.0f) {
         addPos<COMP>(V, i, v3(V.g->kin[i]), h);  // prescribed motion
         return;
@@ -856,7 +859,7 @@ __device__ __forceinline__ void predictParticleFrom(const RodView& V, int i, flo
 
 template <bool COMP>
 __device__ __forceinline__ void predictParticle(const RodView& V, int i, float h, V3 g) {
-    predictParticleFrom<COMP>(V, i, V.g->invMass[i], h, g, V.v[i], &V.v[i]);
+    predictParticleFrom<COMP>(V, i, h, g, V.v[i], &V.v[i]);
 }
 
 // Prediction of frame j from the angular velocity wIn (*wOut as for the
@@ -896,15 +899,15 @@ __device__ __forceinline__ void predictFrame(const RodView& V, int j, float h) {
 // Velocity of particle i at the end of a substep (recovered from its
 // displacement; a kinematic particle takes its prescribed velocity).
 template <bool COMP>
-__device__ __forceinline__ float4 finishedVelocity(const RodView& V, int i, float w, float h, float linDecay) {
-    if (w == 0.0f) return V.g->kin[i];
+__device__ __forceinline__ float4 finishedVelocity(const RodView& V, int i, float h, float linDecay) {
+    if (V.x[i].w == 0.0f) return V.g->kin[i];
     const V3 d = dispOf<COMP>(V, i);
     return f4(divs(d, h) * linDecay);
 }
 
 template <bool COMP>
 __device__ __forceinline__ void finishParticle(const RodView& V, int i, float h, float linDecay) {
-    V.v[i] = finishedVelocity<COMP>(V, i, V.xPrev[i].w, h, linDecay);
+    V.v[i] = finishedVelocity<COMP>(V, i, h, linDecay);
 }
 
 // Angular velocity of frame j at the end of a substep (from the substep's
