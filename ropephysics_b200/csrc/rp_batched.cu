@@ -163,6 +163,7 @@ constexpr int kMaxWarps = 16;  // of a CTA
 // would be a generic load.
 struct TeamCtx {
     RodGlobals G;                   // the rod's fixed global pointers (V.g)
+    float4 rows[5];                 // its template rows where they are all equal
     RodView V;                      // copies of the view and scratch for the
     SelfScratch S;                  // separately compiled paths
     float4* velocity;               // the rod's velocities in global memory
@@ -835,6 +836,15 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
         G.bComp = A.tBComp + T.bOff;
         G.bRestD = A.tBRestD + T.bOff;
         G.prims = A.prims + R.primOff;
+        if (V.rowMask == 0) {
+            const float4* const from[5] = {G.invInertia, G.inertia, G.sComp, G.bComp, G.bRestD};
+            for (int i = 0; i < 5; ++i) C.rows[i] = i < 3 || nB > 0 ? *from[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            G.invInertia = &C.rows[0];
+            G.inertia = &C.rows[1];
+            G.sComp = &C.rows[2];
+            G.bComp = &C.rows[3];
+            G.bRestD = &C.rows[4];
+        }
         // lean layout: loads and kinematic velocities stay in global memory
         G.force = A.force + R.pOff;
         G.kin = A.kinVel + R.pOff;

@@ -68,7 +68,7 @@ struct RodLayout {
 //   batched kernel, whose teams may have 16 warps
 constexpr int32_t kMiscBytes = 320;
 constexpr int32_t kMiscBytesLong = 576;
-constexpr int32_t kContextBytes = 496;
+constexpr int32_t kContextBytes = 576;
 
 // Shared memory of one self contact while it is projected (batched kernel):
 // five 8-byte rows. A pool of nSt / 2 of them is the 20 nSt bytes that the

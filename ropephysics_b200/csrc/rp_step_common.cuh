@@ -168,8 +168,8 @@ template <bool COMP>
 __device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int i0, int i1, int j) {
     const RodView& V = *g->view;
     const float w0 = V.g->invMass[i0], w1 = V.g->invMass[i1];
-    const V3 iI = v3(V.g->invInertia[j]);
-    const float4 sc = V.g->sComp[k];
+    const V3 iI = v3(V.g->invInertia[j & V.rowMask]);
+    const float4 sc = V.g->sComp[k & V.rowMask];
     const float l = sc.w;
     const Q4 q = q4(V.q[j]);
     V3 d = v3(V.x[i1]) - v3(V.x[i0]);
@@ -274,13 +274,13 @@ __device__ __forceinline__ void projectStretchOne(const RodView& V, int k) {
 template <bool COMP>
 __device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a, int b) {
     const RodView& V = *g0->view;
-    const V3 iIa = v3(V.g->invInertia[a]), iIb = v3(V.g->invInertia[b]);
-    const float4 bc = V.g->bComp[k];
+    const V3 iIa = v3(V.g->invInertia[a & V.rowMask]), iIb = v3(V.g->invInertia[b & V.rowMask]);
+    const float4 bc = V.g->bComp[k & V.rowMask];
     const float lbar = bc.w;
     const Q4 qa = q4(V.q[a]);
     const Q4 qb = q4(V.q[b]);
     const Q4 p = sameHemisphereId(qmulConj(qa, qb));
-    const V3 C = fmav(im(p), 2.0f / lbar, -v3(V.g->bRestD[k]));
+    const V3 C = fmav(im(p), 2.0f / lbar, -v3(V.g->bRestD[k & V.rowMask]));
 
     const M3 skewPv = mskew(im(p));
     const M3 Ja = mscale(madd(midentity(-p.w), skewPv), 1.0f / lbar);
