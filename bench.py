@@ -674,11 +674,14 @@ def run_ours(args):
         line["served"] = run_served(value, args.served_seconds, args.seed + 7,
                                     args.served_load, args.served_budget_gb)
     if rank == 0 and world_size == 1 and not args.no_cpu:
-        rate, kind, sample, threads = cpu_reference_rate(args.workload, args.rods, args.seed, args.cpu_rods,
-                                                          args.cpu_seconds, os.cpu_count() or 1,
-                                                          args.warmup + args.steps)
-        line["cpu_baseline"] = {"value": rate, "unit": "segment-substeps/s", "cores": threads,
-                                "kind": kind, "sample": sample}
+        try:
+            rate, kind, sample, threads = cpu_reference_rate(args.workload, args.rods, args.seed, args.cpu_rods,
+                                                              args.cpu_seconds, os.cpu_count() or 1,
+                                                              args.warmup + args.steps)
+            line["cpu_baseline"] = {"value": rate, "unit": "segment-substeps/s", "cores": threads,
+                                    "kind": kind, "sample": sample}
+        except FileNotFoundError as e:  # the reference is not built here
+            line["cpu_baseline"] = {"unavailable": str(e)}
     if rank == 0:
         print(json.dumps(line), flush=True)
     batch.close()
@@ -803,7 +806,11 @@ def run_reference(args):
     config = workload_config(args.workload, args.rods, args.seed)
     config["parallelism"] = f"replicas{world_size}"
     threads = os.cpu_count() or 1
-    sample = ReferenceSample(args.workload, args.rods, args.seed, args.cpu_rods)
+    try:
+        sample = ReferenceSample(args.workload, args.rods, args.seed, args.cpu_rods)
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     # warm-up: advance the sample to the step the GPU arm's timed region
     # starts at (its warm-up steps plus its graph warm-up of `steps` steps)
     sample.run(max(1, args.warmup + args.steps), threads)
