@@ -50,9 +50,9 @@ FLOPS_PER_SEG_SUBSTEP = {"uneven": 1696.2, "hook": 1446.1, "grid": 890.5, "canti
 # float4 rows): read 4 x 16 + 3 x 16, written 2 x 16 + 2 x 16.
 BYTES_PER_SEG_STEP = 7 * 16 + 4 * 16
 # Measured DRAM bytes (read + write) per segment-step of the batched step,
-# from one ncu capture of a 4096-rod uneven batch (state beyond L2, so the
-# figure scales with segments: 246.0 MB over 1 084 256 segments).
-DRAM_BYTES_PER_SEG_STEP = {"uneven": 226.9}
+# from one ncu capture of the 16384-rod uneven batch (724.4 MB over 4 340 093
+# segments; equal template rows are read once per rod, not per segment).
+DRAM_BYTES_PER_SEG_STEP = {"uneven": 166.9}
 
 
 def measured_peaks():
@@ -660,7 +660,7 @@ def run_ours(args):
                      "note": "of measured: peak = FP32 FMA microkernel on this GPU (rp_measure_fp32_peak); "
                              "FLOPs = the reference step's add/sub/mul/div/sqrt count on this workload "
                              "(op-counting oracle, contacts and self-collision included); traffic = DRAM "
-                             "bytes per launch from ncu on 4096 rods, scaled by segments"},
+                             "bytes per launch from ncu on the 16384-rod batch, by segments"},
         "hbm": {"achieved": bytes_launch / per_launch_s / 1e9, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                 "frac": bytes_launch / per_launch_s / 1e9 / peaks.get("hbm_gbs", 6650.0),
                 "bytes_per_segment_step": BYTES_PER_SEG_STEP,
