@@ -297,9 +297,11 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
     // they are, a segment per lane. The others need no test where the centres 8
     // and 18 segments on lie so far from j that those before and shortly
     // behind them, each at most the longest segment from the next, are out of
-    // reach as well (the factor 1.002 is far above the rounding). A gap above 7
-    // is past what this covers: such rods test all near pairs.
-    const bool split = gap < 8;
+    // reach as well (the factor 1.002 is far above the rounding). That is so
+    // on a chain only: segments of consecutive indices lie anywhere in other
+    // rods, which test all near pairs, and so do rods with a gap above 7, past
+    // what this covers.
+    const bool split = C.chain && gap < 8;
     const int near = split ? gap + 1 : gap;
     const int last = nSt - 1;
     const float step = (cell - 2.0f * C.V.g->radius) * 1.0001f;  // the longest segment
