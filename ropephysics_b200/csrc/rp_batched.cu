@@ -1102,9 +1102,11 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
                 predictFrameFrom<COMP>(V, j, h, wj, nullptr);
             }
             teamSync(team, teamIdx);
-            // the ordered pool into shared memory, read again only after the
-            // barriers of the sweeps below
-            if (self && regenerate && *numLevels > 0)
+            // the ordered pool into shared memory, over the count's centres and
+            // counts: the barriers of the sweeps below come before its rows are
+            // read and before the next substep's centre pass writes there again.
+            // A step of no sweeps has no such barrier, and nothing reads the rows.
+            if (self && regenerate && A.iterations > 0 && *numLevels > 0)
                 for (int c = lane; c < *S.live; c += team) compactContact(S, c, *S.live);
 
             for (int it = 0; it < A.iterations; ++it) {
