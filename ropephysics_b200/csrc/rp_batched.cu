@@ -391,8 +391,9 @@ static_assert(sizeof(TeamCtx) <= kContextBytes && alignof(TeamCtx) <= 16, "the l
 // 35 % of the step of 32 settled rods of 1500-2200 segments (474 contacts in
 // 55 levels).
 //
-// An entry that indexes outside the rod or was left unwritten cuts the pool
-// before it and is reported; it is never dereferenced.
+// An entry that was left unwritten (its id is -1 until the thread that writes
+// the entry sets it) or that indexes outside the rod cuts the pool before it and
+// is reported; it is never dereferenced.
 __device__ __forceinline__ void orderPool(const TeamCtx& C, int live, int precision, int32_t* errorWord, int lane) {
     constexpr unsigned kAll = 0xffffffffu;
     const SelfScratch& S = C.S;
@@ -583,6 +584,7 @@ __device__ __forceinline__ int poolFromPairs(const TeamCtx& C, int numPairs, int
     }
     const int total = __reduce_add_sync(0xffffffffu, __popc(cells));
     __syncwarp();
+    for (int c = lane; c < min(total, C.selfCapacity); c += 32) ids[c] = -1;  // not written yet
     if (mine) S.segCount[lane] = int32_t(cells);
     __syncwarp();
     if (mine) {
@@ -638,6 +640,7 @@ __device__ __forceinline__ int poolFromManyPairs(const TeamCtx& C, int numPairs,
         cellsOf[p] = S.sorted[p];
     }
     const int total = teamExclusiveScan(S.segCount, nSt, lane, team, teamIdx, C.partial());
+    for (int c = lane; c < min(total, C.selfCapacity); c += team) ids[c] = -1;  // not written yet
     for (int p = lane; p < numPairs; p += team) next[p] = atomicExch(&head[S.segStart[p] >> 16], p);
     teamSync(team, teamIdx);
     for (int p = lane; p < numPairs; p += team) {
