@@ -317,6 +317,9 @@ __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfSc
             const float need18 = (reach + float(max(e18 - j - 13, e18 < last ? 5 : 0)) * step) * 1.002f;
             clear = __ballot_sync(0xffffffffu, (e8 - j < near || d8 > need8 * need8) &&
                                                    (e18 - j < 13 || d18 > need18 * need18));
+            // a centre that is no number says nothing of its neighbours' places
+            // (the centres read here are all that the chunk's near pairs have)
+            if (__any_sync(0xffffffffu, !(d8 + d18 >= 0.0f))) clear = 0u;
         }
         if (clear == 0xffffffffu) continue;
 #pragma unroll 1
