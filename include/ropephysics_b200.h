@@ -359,11 +359,17 @@ rp_status rp_batch_set_graph(rp_batch* batch, int32_t enabled);
  * CTA = CTA size / team size), pairs per thread (a rod of n segments gets a
  * team of about n / (2 x pairs) threads, whole warps, 32..256) and whole steps
  * per launch in rp_batch_step_many. None of them changes results.
+ * A batch whose shape nobody set reports 256 threads and one pair per thread and
+ * runs that shape, except where all its rods together leave half the GPU's
+ * threads idle: then its longest rods get teams of about n threads, up to 512,
+ * in CTAs of 128, 256 or 512. A shape given to rp_batch_set_tuning, 256 and 1
+ * included, is run as given.
  * cta_threads 0 selects one rod per CTA with every array staged in shared
  * memory (the RP_STRATEGY_FUSED kernel, same results), which wins for a few
  * short rods; it needs each rod's full layout to fit one CTA.
  * rp_batch_autotune times the candidate shapes on this batch with its current
- * state (restored afterwards) and keeps the fastest; steps per launch is
+ * state (restored afterwards), the one of a batch nobody tuned among them
+ * (again reported as 256 and 1), and keeps the fastest; steps per launch is
  * tried up to max_steps_per_launch (at most 8), then one rod per CTA. */
 rp_status rp_batch_autotune(rp_batch* batch, const rp_step_params* params, int32_t max_steps_per_launch);
 rp_status rp_batch_get_tuning(const rp_batch* batch, int32_t* cta_threads, int32_t* pairs_per_thread,

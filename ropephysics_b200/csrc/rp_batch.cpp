@@ -382,7 +382,8 @@ rp_status buildBatchedPlan(rp_batch* b, const Tune& tune, int precision) {
     for (int r = 0; r < b->numRods; ++r) ids[r] = r;
     rpx::BatchedShape shape;
     const rp_status planned = rpx::planBatched(ids, b->rods.data(), b->tmpls.data(), tune.ctaThreads,
-                                               tune.pairsPerThread, precision, b->device, b->maxPrims > 0, shape);
+                                               tune.pairsPerThread, tune.mayWiden, precision, b->device,
+                                               b->maxPrims > 0, shape);
     if (planned != RP_OK) return planned;
     std::vector<int32_t>&order = shape.order, &groups = shape.groups;
     const int numGroups = int(groups.size() / 4);
@@ -436,6 +437,8 @@ rp_status buildBatchedPlan(rp_batch* b, const Tune& tune, int precision) {
     b->batchedBlocks = shape.blocks;
     b->tune.ctaThreads = tune.ctaThreads;
     b->tune.pairsPerThread = tune.pairsPerThread;
+    b->tune.mayWiden = tune.mayWiden;
+    b->batchedWide = shape.wide;
     return RP_OK;
 }
 
@@ -816,8 +819,9 @@ rp_status rp_batch_set_tuning(rp_batch* b, int32_t cta_threads, int32_t pairs_pe
     want.ctaThreads = cta_threads;
     want.pairsPerThread = pairs_per_thread;
     want.stepsPerLaunch = steps_per_launch;
+    want.mayWiden = false;  // the shape asked for, as it is
     want.plain = false;
-    if (want.ctaThreads != b->tune.ctaThreads || want.pairsPerThread != b->tune.pairsPerThread) {
+    if (want.ctaThreads != b->tune.ctaThreads || want.pairsPerThread != b->tune.pairsPerThread || b->batchedWide) {
         if ((st = buildBatchedPlan(b, want, b->precision)) != RP_OK) return st;  // batch unchanged
     }
     b->tune = want;

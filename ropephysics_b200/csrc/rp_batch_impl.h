@@ -33,6 +33,8 @@ struct Tune {
     int ctaThreads = 256;     // threads per CTA (rods per CTA = ctaThreads / team)
     int pairsPerThread = 1;   // team threads ~ ceil(nSt / 2 / pairsPerThread), rounded to 32
     int stepsPerLaunch = 1;   // whole steps (x substeps) per launch in rp_batch_step_many
+    bool mayWiden = true;     // no shape was asked for: small launches may take wide
+                              // teams instead (planBatched)
     bool plain = false;       // one rod per CTA, every array staged: the plain kernel
                               // (RP_STRATEGY_FUSED's), faster for a few short rods
 };
@@ -74,6 +76,7 @@ struct rp_batch {
     int32_t* dQueue = nullptr;
     int numGroups = 0;
     int batchedBlocks = 0;
+    bool batchedWide = false;  // the plan has wide teams instead of the tuned shape
     int batchedThreads = 256;
     size_t batchedSmem = 0;
     rpx::Tune tune;

@@ -113,26 +113,33 @@ rp_status rp_batch_autotune(rp_batch* b, const rp_step_params* p, int32_t max_st
     b->tune.plain = false;  // the batched shapes first
     float bestMs = 3.0e38f;
     // rods per CTA and threads per rod: every (CTA size, team size) pair that
-    // plans, one warm launch and two timed launches from the same state
-    for (int cta : {128, 256}) {
-        for (int ppt : {1, 2}) {
-            Tune trialShape = best;
-            trialShape.ctaThreads = cta;
-            trialShape.pairsPerThread = ppt;
-            trialShape.stepsPerLaunch = 1;
-            if (buildBatchedPlan(b, trialShape, b->precision) != RP_OK) continue;
-            b->tune.stepsPerLaunch = 1;
-            float ms = 0.0f;
-            if ((st = snap.restore(b)) != RP_OK) break;
-            if ((st = launchStep(b, p, 1)) != RP_OK) break;
-            if ((st = snap.restore(b)) != RP_OK) break;
-            if ((st = timeSteps(b, p, 1, 2, &ms)) != RP_OK) break;
-            if (ms < bestMs) {
-                bestMs = ms;
-                best = b->tune;
-            }
+    // plans, and the plan of a batch nobody tuned where that is another one (wide
+    // teams); one warm launch and two timed launches each from the same state
+    const struct {
+        int cta, ppt;
+        bool mayWiden;
+    } shapes[] = {{128, 1, false}, {128, 2, false}, {256, 1, true}, {256, 1, false}, {256, 2, false}};
+    bool widened = false;
+    for (const auto& shape : shapes) {
+        if (shape.cta == 256 && shape.ppt == 1 && !shape.mayWiden && !widened) continue;  // timed already
+        Tune trialShape = best;
+        trialShape.ctaThreads = shape.cta;
+        trialShape.pairsPerThread = shape.ppt;
+        trialShape.mayWiden = shape.mayWiden;
+        trialShape.stepsPerLaunch = 1;
+        const rp_status planned = buildBatchedPlan(b, trialShape, b->precision);
+        if (shape.mayWiden) widened = planned == RP_OK && b->batchedWide;
+        if (planned != RP_OK) continue;
+        b->tune.stepsPerLaunch = 1;
+        float ms = 0.0f;
+        if ((st = snap.restore(b)) != RP_OK) break;
+        if ((st = launchStep(b, p, 1)) != RP_OK) break;
+        if ((st = snap.restore(b)) != RP_OK) break;
+        if ((st = timeSteps(b, p, 1, 2, &ms)) != RP_OK) break;
+        if (ms < bestMs) {
+            bestMs = ms;
+            best = b->tune;
         }
-        if (st != RP_OK) break;
     }
     // whole steps per launch, on the chosen shape; a longer launch must win
     // by 2 % to be kept

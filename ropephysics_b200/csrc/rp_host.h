@@ -59,9 +59,11 @@ struct BatchedShape {
     size_t smem = 0;                     // dynamic shared memory per CTA
     int slotsShared = 0;                 // world contact slots in shared memory
     bool anySelf = false;                // a rod collides with itself
+    bool wide = false;                   // wide teams instead of the asked shape
 };
 rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
-                      int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out);
+                      int pairsPerThread, bool mayWiden, int precision, int device, bool mayShareSlots,
+                      BatchedShape& out);
 
 // ---- rp_batch.cpp: what the trajectory writer reads of a batch ----
 struct BatchView {

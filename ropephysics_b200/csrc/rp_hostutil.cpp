@@ -319,7 +319,8 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
 }  // namespace
 
 // The launch of the batched kernel over `rodIds` with the asked CTA size and
-// segment pairs per thread.
+// segment pairs per thread, or, with `mayWiden` (nobody asked for a shape), with
+// wide teams where the launch leaves room for them.
 //
 // The default shape (256 threads, one pair per thread) gives a rod the threads
 // its constraint colours need, which is best while the GPU is full. With fewer
@@ -337,13 +338,14 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
 // 16 of 900 295 -> 222 (112 -> 84), 64 settled rods of 40-200 with
 // self-collision 1271 -> 968 (447 -> 355).
 rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
-                      int pairsPerThread, int precision, int device, bool mayShareSlots, BatchedShape& out) {
+                      int pairsPerThread, bool mayWiden, int precision, int device, bool mayShareSlots,
+                      BatchedShape& out) {
     const size_t optin = optinSmem(device);
     int sms = 0, perSm = 0;
-    out.anySelf = false;
+    out.anySelf = out.wide = false;
     for (int32_t r : rodIds) out.anySelf = out.anySelf || rods[r].selfCollision != 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (cta == 256 && pairsPerThread == 1) {
+    if (mayWiden) {
         int longest = 0;
         for (int32_t r : rodIds) longest = std::max(longest, tmpls[rods[r].tmpl].nSt);
         for (int wideFrom = 0; wideFrom < std::min(longest, 449); wideFrom += 64) {
@@ -360,6 +362,7 @@ rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, 
                     RP_OK &&
                 int(out.groups.size() / 4) <= sms * perSm) {
                 out.blocks = std::max(1, int(out.groups.size() / 4));
+                out.wide = true;
                 return RP_OK;
             }
         }

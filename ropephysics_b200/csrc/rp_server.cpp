@@ -316,7 +316,8 @@ bool rp_server::plan() {
     std::vector<int32_t> ids;
     for (auto& rq : running) ids.insert(ids.end(), rq->rodIds.begin(), rq->rodIds.end());
     rpx::BatchedShape shape;
-    if (rpx::planBatched(ids, hRods.data(), hTmpls.data(), 256, 1, cfg.precision, device, false, shape) != RP_OK) {
+    if (rpx::planBatched(ids, hRods.data(), hTmpls.data(), 256, 1, true, cfg.precision, device, false, shape) !=
+        RP_OK) {
         workerError = rp_last_error();
         return false;
     }
