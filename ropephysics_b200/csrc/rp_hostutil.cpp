@@ -228,10 +228,10 @@ int teamThreads(int nSt, bool self, int pairsPerThread, int wideFrom) {
 // would break the 16-byte alignment its rows and bulk copies need: refused
 // on the host, never launched). `order` receives the rod ids
 // longest first (stable), `groups` four ints per group: first index into
-// `order`, rod count, team size, shared bytes. Returns the largest group's
-// shared bytes.
+// `order`, rod count, team size, shared bytes. A group ends before the rod that
+// would take it past `room` bytes. Returns the largest group's shared bytes.
 size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls,
-                  int cta, int pairsPerThread, int wideFrom, bool comp, bool slotsShared,
+                  int cta, int pairsPerThread, int wideFrom, bool comp, bool slotsShared, size_t room,
                   std::vector<int32_t>& order, std::vector<int32_t>& groups) {
     order = rodIds;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
@@ -257,6 +257,7 @@ size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, cons
                                                   R.hashTableSize, R.selfCapacity, 1, comp ? 1 : 0,
                                                   slotsShared ? 1 : 0);
             if (!rp::rodLayoutAligned(L)) return kMisaligned;
+            if (cnt > 0 && smem + size_t(L.bytes) > room) break;
             smem += size_t(L.bytes);
             ++cnt;
         }
@@ -279,7 +280,8 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
     const size_t fixed = rp::batchedStaticSmem() + 64;  // the kernel's own shared memory
     out.cta = cta;
     out.slotsShared = 0;
-    out.smem = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, false, out.order, out.groups);
+    const size_t room = fixed < optin ? optin - fixed : 0;
+    out.smem = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, false, room, out.order, out.groups);
     if (out.smem == kMisaligned)
         return fail(RP_ERR_INVALID, "internal: a rod's shared-memory layout is not 16-byte aligned");
     // World contact slots go into shared memory when the groups still fit as
@@ -287,8 +289,8 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
     // rods); otherwise they stay in global memory.
     if (mayShareSlots) {
         std::vector<int32_t> order2, groups2;
-        const size_t smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, order2,
-                                        groups2);
+        const size_t smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, SIZE_MAX,
+                                        order2, groups2);
         int per1 = 0, per2 = 0;
         if (smem2 != kMisaligned && smem2 + fixed <= optin &&
             rp::batchedReserveSmem(std::max(smem2, out.smem)) == cudaSuccess &&
