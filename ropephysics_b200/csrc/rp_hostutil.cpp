@@ -271,11 +271,23 @@ size_t planGroups(const std::vector<int32_t>& rodIds, const rp::DRod* rods, cons
     return maxSmem;
 }
 
+// Shared memory of a CTA if an SM is to hold `ctas` of them.
+size_t smemPerCta(int device, int ctas) {
+    int sm = 0, reserved = 0;
+    if (cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return size_t(std::max(0, sm / ctas - reserved));
+}
+
 // One launch shape: its groups, its shared memory, and how many of its CTAs
 // an SM holds.
 rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
-                    int pairsPerThread, int wideFrom, int precision, size_t optin, bool mayShareSlots,
+                    int pairsPerThread, int wideFrom, int precision, int device, bool mayShareSlots,
                     BatchedShape& out, int* perSm) {
+    const size_t optin = optinSmem(device);
     const bool comp = (precision & RP_PRECISION_COMPENSATED) != 0;
     const size_t fixed = rp::batchedStaticSmem() + 64;  // the kernel's own shared memory
     out.cta = cta;
@@ -286,22 +298,41 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
         return fail(RP_ERR_INVALID, "internal: a rod's shared-memory layout is not 16-byte aligned");
     // World contact slots go into shared memory when the groups still fit as
     // many CTAs per SM with them (few contact primitives per rod, or short
-    // rods); otherwise they stay in global memory.
+    // rods); otherwise they stay in global memory. Where only the teams' contexts
+    // take them past that, the groups give up a rod and keep the slots: 4096 rods
+    // of 60 lying on their primitives (five a rod), 20 substeps, take 906 us with
+    // eight to a CTA and the slots in global memory and 519 with seven. Far from
+    // the primitives, where no slot is touched, it is 281 and 290 (2100 rods of
+    // 61, a last wave more: 149 and 240).
     if (mayShareSlots) {
         std::vector<int32_t> order2, groups2;
-        const size_t smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, SIZE_MAX,
-                                        order2, groups2);
-        int per1 = 0, per2 = 0;
-        if (smem2 != kMisaligned && smem2 + fixed <= optin &&
-            rp::batchedReserveSmem(std::max(smem2, out.smem)) == cudaSuccess &&
-            rp::batchedOccupancy(cta, out.smem, precision, out.anySelf, &per1) == cudaSuccess &&
-            rp::batchedOccupancy(cta, smem2, precision, out.anySelf, &per2) == cudaSuccess && per2 >= per1 && per2 >= 1) {
+        size_t smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, SIZE_MAX, order2,
+                                  groups2);
+        auto ctas = [&](size_t smem) {  // an SM holds
+            int n = 0;
+            if (smem + fixed > optin || rp::batchedReserveSmem(std::max<size_t>(smem, 1)) != cudaSuccess ||
+                rp::batchedOccupancy(cta, smem, precision, out.anySelf, &n) != cudaSuccess)
+                n = 0;
+            cudaGetLastError();
+            return n;
+        };
+        const int most = smem2 == kMisaligned ? 0 : ctas(out.smem);
+        if (most >= 1 && ctas(smem2) < most) {
+            size_t bare = 0;  // the largest group without its contexts
+            for (size_t g = 0; g < groups2.size(); g += 4)
+                bare = std::max(bare, size_t(groups2[g + 3]) - size_t(groups2[g + 1]) * rp::kContextBytes);
+            const size_t each = smemPerCta(device, most);
+            const size_t room2 = std::min(room, each > fixed ? each - fixed : 0);
+            if (bare <= room2)
+                smem2 = planGroups(rodIds, rods, tmpls, cta, pairsPerThread, wideFrom, comp, true, room2, order2,
+                                   groups2);
+        }
+        if (most >= 1 && ctas(smem2) >= most) {
             out.smem = smem2;
             out.order.swap(order2);
             out.groups.swap(groups2);
             out.slotsShared = 1;
         }
-        cudaGetLastError();
     }
     if (out.smem + fixed > optin)
         return fail(RP_ERR_SHARED_MEMORY, "a rod group needs " + std::to_string(out.smem) +
@@ -342,7 +373,6 @@ rp_status planShape(const std::vector<int32_t>& rodIds, const rp::DRod* rods, co
 rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, const rp::DTemplate* tmpls, int cta,
                       int pairsPerThread, bool mayWiden, int precision, int device, bool mayShareSlots,
                       BatchedShape& out) {
-    const size_t optin = optinSmem(device);
     int sms = 0, perSm = 0;
     out.anySelf = out.wide = false;
     for (int32_t r : rodIds) out.anySelf = out.anySelf || rods[r].selfCollision != 0;
@@ -360,7 +390,7 @@ rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, 
             }
             if (threads > int64_t(sms) * 256) continue;
             const int wideCta = most <= 128 ? 128 : most <= 256 ? 256 : 512;
-            if (planShape(rodIds, rods, tmpls, wideCta, 1, wideFrom, precision, optin, mayShareSlots, out, &perSm) ==
+            if (planShape(rodIds, rods, tmpls, wideCta, 1, wideFrom, precision, device, mayShareSlots, out, &perSm) ==
                     RP_OK &&
                 int(out.groups.size() / 4) <= sms * perSm) {
                 out.blocks = std::max(1, int(out.groups.size() / 4));
@@ -369,7 +399,7 @@ rp_status planBatched(const std::vector<int32_t>& rodIds, const rp::DRod* rods, 
             }
         }
     }
-    const rp_status st = planShape(rodIds, rods, tmpls, cta, pairsPerThread, kNoWide, precision, optin, mayShareSlots,
+    const rp_status st = planShape(rodIds, rods, tmpls, cta, pairsPerThread, kNoWide, precision, device, mayShareSlots,
                                    out, &perSm);
     if (st == RP_OK) out.blocks = std::max(1, std::min(int(out.groups.size() / 4), sms * perSm));
     return st;
