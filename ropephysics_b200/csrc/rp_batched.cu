@@ -31,7 +31,8 @@
 //     particle), which reproduces the sequential order's arithmetic, from
 //     shared memory and by one warp while levels are narrow.
 // Every per-element operation is the shared code in rp_step_common.cuh, so
-// results are bit-identical to the plain kernel.
+// results are bit-identical to the plain kernel (contacts of a rod with itself
+// use shared reciprocals here; rp_math.cuh names the one tie they round otherwise).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -205,27 +206,7 @@ struct TeamCtx {
     __device__ int32_t* lvlOf() const { return lvlStart() + (selfCapacity + 1); }
 };
 
-// segCount[j] (zeroed by the caller) += the reference's count of segment j;
-// every touching pair (j, k) is also appended to S.segStart as (j << 16) | k
-// (*C.numPairs(), zeroed by the caller, counts them; entries past nSt are not
-// stored).
-// `reach` is the longest segment plus 2 r with the margins of the sphere test
-// of querySelfSegment (1.001 and 1e-6 of the coordinates' size, here of the
-// rod's largest), so a pair whose centres are farther apart fails that test;
-// `cell` is the longest segment plus 2 r. Pairs near along the chain are tested a segment per
-// lane, or ruled out by two distances; the others by chain blocks of 8
-// segments: box distance, then, for blocks within reach, the 64 pairs, two
-// per lane. Box and centre distances are monotone in float, so no pair the
-// sphere test keeps is missed. Pairs within reach wait in the warp's queue,
-// and the narrow phase runs on 32 of them at once.
-//
-// Bound: issue slots. In free fall three of five rounds a block went to near
-// pairs, which no rod passes that is not sharply bent. In settled rods two or
-// three lanes of a round pass, and the narrow phase run for those alone took
-// most of the count. 4096 uneven rods in free fall, 50 substeps, 6.55 -> 5.68 ms
-// (the count 10.6 -> 6.3 thousand cycles a rod and substep); 256 settled rods of
-// 16-512 2.02 -> 1.74 ms; 8 cables of 40-200, 20 substeps, 217 -> 157 us.
-// A pair that passed the sphere test: the shared narrow phase, and for a
+// A pair within reach: the shared narrow phase, and for a
 // touching pair its bucket multiplicity, its count and its place in the pair
 // list (which holds nSt pairs; beyond that the count alone is kept and the
 // pool is built from the hash). Not inlined: few pairs get here, and its
@@ -249,6 +230,28 @@ __device__ __noinline__ void countTouching(const TeamCtx& C, int j, int k, float
     }
 }
 
+// segCount[j] (zeroed by the caller) += the reference's count of segment j;
+// every touching pair (j, k) is also appended to S.segStart as (j << 16) | k
+// (*C.numPairs(), zeroed by the caller, counts them; entries past nSt are not
+// stored).
+// `reach` is the longest segment plus 2 r with the margins of the sphere test
+// of querySelfSegment (1.001 and 1e-6 of the coordinates' size, here of the
+// rod's largest), so a pair whose centres are farther apart fails that test;
+// `cell` is the longest segment plus 2 r. Pairs of near indices are tested a
+// segment per lane, or, on a chain, ruled out by two distances; the others by
+// blocks of 8 segments: box distance, then, for blocks within reach, the 64
+// pairs, two per lane. Box and centre distances are monotone in float, and the
+// two distances bound a chain's centres by its longest segment, so no pair the
+// sphere test keeps is missed (tests/test_count_enumeration.py replays the
+// rounds). Pairs within reach wait in the warp's queue, and the narrow phase
+// runs on 32 of them at once.
+//
+// Bound: issue slots. In free fall three of five rounds a block went to near
+// pairs, which no rod passes that is not sharply bent. In settled rods two or
+// three lanes of a round pass, and the narrow phase run for those alone took
+// most of the count. 4096 uneven rods in free fall, 50 substeps, 6.55 -> 5.68 ms
+// (the count 10.6 -> 6.3 thousand cycles a rod and substep); 256 settled rods of
+// 16-512 2.02 -> 1.74 ms; 8 cables of 40-200, 20 substeps, 217 -> 157 us.
 __device__ __forceinline__ void countSelfByBlocks(const TeamCtx& C, const SelfScratch& S, int nSt, int gap,
                                                   float cell, float reach, int lane, int team) {
     __shared__ int32_t queues[kMaxWarps][32];  // per warp: pairs that wait for the narrow phase
@@ -511,50 +514,50 @@ __device__ __forceinline__ void orderPool(const TeamCtx& C, int live, int precis
 // reference's hash (a stable counting sort) and its fill pass in bucket order.
 // For pools that the pair list cannot give (more than nSt touching pairs).
 __device__ __forceinline__ void fillSelfPool(const TeamCtx& C, float cell, int live, int lane, int team,
-                                          int teamIdx) {
+                                             int teamIdx) {
     const RodView& V = C.V;
     const SelfScratch& S = C.S;
     const int nSt = C.nSt, table = C.table;
     int32_t* const cursor = C.cursor();
     int32_t* const partial = C.partial();
-        // ---- fill, in the reference's order: its hash buckets ----
-        for (int t = lane; t <= table; t += team) S.cellStart[t] = 0;
-        for (int c = lane; c < live; c += team) S.pool[c].seg = -1;
-        teamSync(team, teamIdx);
-        for (int j = lane; j < nSt; j += team) {
-            const float4 c = S.centres[j];
-            const int h0 = int(hashCell(cellCoord(c.x, cell), cellCoord(c.y, cell),
-                                        cellCoord(c.z, cell), table));
-            S.cellOf[j] = h0;
-            atomicAdd(&S.cellStart[h0], 1);
-        }
-        teamSync(team, teamIdx);
-        // counts -> starts: cellStart[t] = first slot of bucket t,
-        // cellStart[table] = segment count (the reference's offsets)
-        teamExclusiveScan(S.cellStart, table + 1, lane, team, teamIdx, partial);
-        for (int t = lane; t < table; t += team) cursor[t] = S.cellStart[t];
-        teamSync(team, teamIdx);
-        // stable placement, one warp walking segments in order
-        if (lane < 32) {
-            for (int j0 = 0; j0 < nSt; j0 += 32) {
-                const int j = j0 + lane;
-                const bool valid = j < nSt;
-                const int c = valid ? S.cellOf[j] : -1 - lane;
-                const unsigned peers = __match_any_sync(0xffffffffu, c);
-                const int rank = __popc(peers & ((1u << lane) - 1u));
-                const int start = valid ? cursor[c] : 0;
-                __syncwarp();
-                if (valid) {
-                    S.sorted[start + rank] = j;
-                    if (rank == 0) cursor[c] = start + __popc(peers);
-                }
-                __syncwarp();
+    // ---- fill, in the reference's order: its hash buckets ----
+    for (int t = lane; t <= table; t += team) S.cellStart[t] = 0;
+    for (int c = lane; c < live; c += team) S.pool[c].seg = -1;
+    teamSync(team, teamIdx);
+    for (int j = lane; j < nSt; j += team) {
+        const float4 c = S.centres[j];
+        const int h0 = int(hashCell(cellCoord(c.x, cell), cellCoord(c.y, cell),
+                                    cellCoord(c.z, cell), table));
+        S.cellOf[j] = h0;
+        atomicAdd(&S.cellStart[h0], 1);
+    }
+    teamSync(team, teamIdx);
+    // counts -> starts: cellStart[t] = first slot of bucket t,
+    // cellStart[table] = segment count (the reference's offsets)
+    teamExclusiveScan(S.cellStart, table + 1, lane, team, teamIdx, partial);
+    for (int t = lane; t < table; t += team) cursor[t] = S.cellStart[t];
+    teamSync(team, teamIdx);
+    // stable placement, one warp walking segments in order
+    if (lane < 32) {
+        for (int j0 = 0; j0 < nSt; j0 += 32) {
+            const int j = j0 + lane;
+            const bool valid = j < nSt;
+            const int c = valid ? S.cellOf[j] : -1 - lane;
+            const unsigned peers = __match_any_sync(0xffffffffu, c);
+            const int rank = __popc(peers & ((1u << lane) - 1u));
+            const int start = valid ? cursor[c] : 0;
+            __syncwarp();
+            if (valid) {
+                S.sorted[start + rank] = j;
+                if (rank == 0) cursor[c] = start + __popc(peers);
             }
+            __syncwarp();
         }
-        teamSync(team, teamIdx);
-        for (int j = lane; j < nSt; j += team)
-            if (S.segCount[j] > 0 && S.segStart[j] < C.selfCapacity)
-                querySelfSegment<true>(V, S, j, nSt, C.selfGap, table, C.selfCapacity, C.selfFriction, true);
+    }
+    teamSync(team, teamIdx);
+    for (int j = lane; j < nSt; j += team)
+        if (S.segCount[j] > 0 && S.segStart[j] < C.selfCapacity)
+            querySelfSegment<true>(V, S, j, nSt, C.selfGap, table, C.selfCapacity, C.selfFriction, true);
 }
 
 // Most touching substeps have a handful of touching pairs; for those the
@@ -714,12 +717,13 @@ __device__ __forceinline__ void compactContact(const SelfScratch& S, int c, int 
 
 // The self-contact pool projected level by level: contacts of one level
 // share no particle, and every earlier contact a contact shares a particle
-// with sits in a lower level -- the serial pool order's result, bit for bit.
+// with sits in a lower level -- the serial pool order's result, bit for bit
+// (but for the ties of rp_math.cuh's shared reciprocals).
 // Not inlined: it runs only while contacts are live. Levels are short (nine
 // contacts on average in settled rods) and there are many, so the chain of
 // one contact's loads and arithmetic per level is what it takes: one warp
 // does them without team barriers unless the levels are wider than a warp,
-// from shared memory (`xAt` .. are byte offsets into it).
+// from shared memory.
 template <bool COMP>
 __device__ __noinline__ void projectSelfCompact(const TeamCtx& C, int levels, int live, int lane, int team,
                                                 int teamIdx) {
@@ -1232,9 +1236,9 @@ __device__ void runRod(const DArgs& A, int r, unsigned char* base, int lane, int
 }
 
 // SELF: some rod of the launch collides with itself. Launches without run an
-// instance without that code, which spills 32 bytes where this one spills 336
-// (loads, reference order) at the 128 registers that two 256-thread CTAs leave:
-// 4096 rods of 64 over a floor, 80 substeps, 1.25 -> 1.13 ms.
+// instance without that code, which spills nothing where this one spills 212
+// bytes (loads, reference order) at the 128 registers that two 256-thread CTAs
+// leave: 4096 rods of 64 over a floor, 80 substeps, 1.25 -> 1.13 ms.
 template <bool COMP, bool FP64, bool SELF>
 __global__ void __launch_bounds__(512, 1) kBatchedStep(DArgs A, const int32_t* __restrict__ groups,
                                                        int numGroups, int32_t* queue) {

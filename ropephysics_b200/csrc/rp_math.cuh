@@ -3,7 +3,8 @@
 // The formulas are those of the reference's shared math (src/core/math3.h and
 // src/core/geometry.h), and so is every floating-point operation and its
 // order, so that the results equal the reference's FP32 GPU kernel
-// (src/gpu/gpu_solver.cu) bit for bit. In particular "vector / scalar" is
+// (src/gpu/gpu_solver.cu) bit for bit, but for one tie in the subnormals (see
+// the shared reciprocals). In particular "vector / scalar" is
 // "vector * (1 / scalar)" (math3.h:75-78).
 //
 // The reference is built with nvcc's default FMA contraction, and which
@@ -105,8 +106,10 @@ __device__ __forceinline__ V3 cwise(V3 a, V3 b) { return V3{a.x * b.x, a.y * b.y
 // (tests/test_gpu_shared_reciprocals.py). A subnormal quotient q - r y is off
 // by less than 2^-174 before its one rounding, and no quotient lies nearer a
 // boundary than that without lying on it: only an exact tie, a = b (2k + 1)
-// 2^-150, which needs an even integer b, could round to the other neighbour,
-// 2^-149 away. Outside the ranges -- NaN, infinities, singular matrices --
+// 2^-150, which needs an even integer b, can round to the other neighbour,
+// 2^-149 away and as near to the quotient (seen in one of 24 batches of 64
+// straight rods set in motion; refusing such divisors costs 4 to 10 % of a
+// step). "Bit for bit" below means but for that tie. Outside the ranges -- NaN, infinities, singular matrices --
 // `ok` turns false and the caller falls back to the plain operators. Signs
 // of zero are kept too (b > 0).
 constexpr float kRootLo = 0x1p-100f, kRootHi = 0x1p100f;  // operands of sqrtRecip
@@ -246,7 +249,8 @@ __device__ __forceinline__ bool solveSPD3(const M3& A, V3 b, V3& y) {
 }
 
 // The same solve with shared reciprocals; `ok` stays true only when the
-// result is solveSPD3's (which then returns true), bit for bit.
+// result is solveSPD3's (which then returns true), bit for bit but for the
+// tie that the shared reciprocals' comment names.
 __device__ __forceinline__ V3 solveSPD3Shared(const M3& A, V3 b, bool& ok) {
     const Divisor l00 = rootDivisor(A.m[0][0], ok);
     const float l10 = quotient(A.m[1][0], l00);

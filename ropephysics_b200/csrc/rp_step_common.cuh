@@ -200,9 +200,10 @@ __device__ __noinline__ void projectStretchPlain(const RodGlobals* g, int k, int
     }
 }
 
-// The same projection, bit for bit, with shared reciprocals: everything is
-// computed and range-tested before the first write, and what the test
-// refuses runs projectStretchPlain instead.
+// The same projection, bit for bit but for the subnormal tie that rp_math.cuh
+// names, with shared reciprocals: everything is computed and range-tested
+// before the first write, and what the test refuses runs projectStretchPlain
+// instead.
 //
 // Bound: the latency of one dependent FP32 chain per constraint (four colours
 // of them per sweep, one to four warps per scheduler); the plain operators
@@ -313,8 +314,7 @@ __device__ __noinline__ void projectBendPlain(const RodGlobals* g0, int k, int a
     }
 }
 
-// The same projection, bit for bit, with shared reciprocals (see
-// projectStretchAt).
+// The same projection with shared reciprocals (see projectStretchAt).
 template <bool COMP>
 __device__ __forceinline__ void projectBendAt(const RodView& V, int k, int a, int b) {
     const V3 iIa = v3(V.g->invInertia[a & V.rowMask]), iIb = v3(V.g->invInertia[b & V.rowMask]);
